@@ -135,7 +135,9 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(T* out, const T* y, 
 }
 
 // w[i] = T(w[i] + T(lora[i] * T(alpha))), each step in T's own arithmetic: loadLora<T>
-// (src/lyradiff/kernels/lora/load_lora.cu:6-14).  n8 vectors of 8 elements, then a scalar tail.
+// (src/lyradiff/kernels/lora/load_lora.cu:6-14).  n8 vectors of 8 elements, then a scalar tail.  A thread has two vectors of
+// each operand in flight: the kernel is a pass over memory and bound by the bytes outstanding (38.9 -> 37.9 us at
+// [12288, 3072] bf16 = 6.0 TB/s).
 template<typename T>
 __global__ void __launch_bounds__(256) load_lora_kernel(T* w, const T* lora, size_t n, float alpha)
 {
@@ -146,14 +148,27 @@ __global__ void __launch_bounds__(256) load_lora_kernel(T* w, const T* lora, siz
     const size_t   n8     = n >> 3;
     const size_t   stride = (size_t)gridDim.x * blockDim.x;
     const size_t   tid    = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (size_t vi = tid; vi < n8; vi += stride) {
-        Vec16       o = *reinterpret_cast<const Vec16*>(w + (vi << 3));  // plain load: this kernel writes w
-        const Vec16 l = ld_nc_16(lora + (vi << 3));
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            o.w[j] = P2::add(o.w[j], P2::mul(l.w[j], a2));
+    for (size_t v0 = tid; v0 < n8; v0 += 2 * stride) {
+        const size_t v1   = v0 + stride;
+        const bool   both = v1 < n8;
+        Vec16        o[2], l[2];
+        o[0] = ld_16(w + (v0 << 3));
+        l[0] = ld_nc_16(lora + (v0 << 3));
+        if (both) {
+            o[1] = ld_16(w + (v1 << 3));
+            l[1] = ld_nc_16(lora + (v1 << 3));
         }
-        st_16(w + (vi << 3), o);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                o[q].w[j] = P2::add(o[q].w[j], P2::mul(l[q].w[j], a2));
+            }
+        }
+        st_16(w + (v0 << 3), o[0]);
+        if (both) {
+            st_16(w + (v1 << 3), o[1]);
+        }
     }
     for (size_t i = (n8 << 3) + tid; i < n; i += stride) {
         const T t = from_f32<T>(to_f32(lora[i]) * to_f32(from_f32<T>(alpha)));  // exact product of two T values, one rounding

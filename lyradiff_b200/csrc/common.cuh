@@ -183,6 +183,13 @@ __device__ __forceinline__ uint4 ld_u32x4(const uint4* p)
     return v;
 }
 
+// 16 bytes of memory that the kernel itself writes (no non-coherent load)
+__device__ __forceinline__ Vec16 ld_16(const void* p)
+{
+    Vec16 v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ void st_16(void* p, const Vec16& v)
 {
     asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.w[0]), "r"(v.w[1]), "r"(v.w[2]), "r"(v.w[3])

@@ -1061,21 +1061,38 @@ __global__ void __launch_bounds__(256) fp8_cast_bulk_kernel(uint8_t* dst, const 
     }
 }
 
-// max|w|/448 folded into scale[0] with an integer atomicMax on the (non-negative) float bits.
+// max|w|/448 folded into scale[0] with an integer atomicMax on the (non-negative) float bits.  A pass over the weight and
+// nothing else, so it is bound by the loads in flight: four 16-byte loads per thread (one per thread kept 32 KB per SM
+// outstanding, half of what HBM's latency needs).  The weight is walked from its END: what was written last -- the merge of a
+// LoRA swap runs right in front of this -- is what L2 still holds, and the cast that follows starts with what this pass read last.
+// [12288, 3072] bf16: 15.3 -> 12.7 us (5.9 TB/s), the scale and cast of a whole lyraq_weight_quant_fp8 36.9 -> 32.7 us.
+constexpr int kAmaxTile = 1024;   // vectors of 8 values per block and step
 template<typename T> __global__ void __launch_bounds__(256) fp8_amax_kernel(float* scale, const T* src, size_t n)
 {
     __shared__ float red[8];
     grid_launch_dependents();
     grid_dependency_wait();
-    const size_t     nvec   = n >> 3;
-    const size_t     stride = (size_t)gridDim.x * blockDim.x;
-    float            amax   = 0.0f;
-    for (size_t vi = (size_t)blockIdx.x * blockDim.x + threadIdx.x; vi < nvec; vi += stride) {
-        float v[8];
-        unpack8<T>(ld_nc_16(src + (vi << 3)), v);
+    const size_t nvec  = n >> 3;
+    const size_t tiles = (nvec + kAmaxTile - 1) / kAmaxTile;
+    float        amax  = 0.0f;
+    for (size_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const size_t v0 = (tiles - 1 - t) * kAmaxTile + threadIdx.x;
+        Vec16        x[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            amax = fmaxf(amax, fabsf(v[j]));
+        for (int i = 0; i < 4; ++i) {
+            x[i].w[0] = x[i].w[1] = x[i].w[2] = x[i].w[3] = 0u;
+            if (v0 + 256 * i < nvec) {
+                x[i] = ld_nc_16(src + ((v0 + 256 * i) << 3));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float v[8];
+            unpack8<T>(x[i], v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                amax = fmaxf(amax, fabsf(v[j]));
+            }
         }
     }
     if (blockIdx.x == 0 && threadIdx.x < (n & 7)) {

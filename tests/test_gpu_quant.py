@@ -142,6 +142,31 @@ def test_fp8_weight_quant_in_one_call(ops, dtype):
     assert_bit_equal(q, quant.fp8_quant(w, want_s, invert_scale=True))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 2047, 2048, 8191, 8192, 8193, 8192 * 3 + 8, 8192 * 1300 + 5])
+def test_fp8_weight_amax_finds_the_maximum_wherever_it_lies(ops, dtype, n):
+    """Around the edges of the amax kernel's steps (1024 vectors of 8 values, the scalar tail): the largest magnitude first,
+    last and at the borders of a step, against a background that is smaller; a maximum is exact."""
+    for at in sorted({0, n - 1, n // 2, min(n - 1, 8191), min(n - 1, 8192), max(0, n - 9)}):
+        w = torch.full((n,), 0.25, dtype=dtype, device="cuda")
+        w[at] = -1.75
+        s = torch.zeros(1, dtype=torch.float32, device="cuda")
+        ops.invoke_get_fp8_weight_scale(s, w)
+        assert float(s) == float(torch.tensor(1.75) / torch.tensor(448.0)), (n, at)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n", [5, 8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 8, 148 * 8 * 256 * 16 + 2043])
+def test_load_lora_around_the_two_vector_step(ops, dtype, n):
+    """One and two vectors per thread, the step's remainder and the scalar tail: the bits of the 16-bit operators."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    w = torch.randn(n, generator=g, device="cuda").to(dtype)
+    lora = torch.randn(n, generator=g, device="cuda").to(dtype)
+    want = (w.float() + (lora.float() * float(torch.tensor(0.7).to(dtype))).to(dtype).float()).to(dtype)
+    ops.invoke_load_lora(w, lora, 0.7)
+    assert torch.equal(w.view(torch.int16), want.view(torch.int16))
+
+
 def test_fp8_weight_quant_reads_its_scale_after_the_amax_kernel(ops):
     """The cast of lyraq_weight_quant_fp8 may start while the amax kernel in front of it still runs (programmatic
     dependent launch) and must read the scale only once that kernel has finished; an early read sees the zero the scale
