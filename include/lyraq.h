@@ -210,9 +210,11 @@ enum {
     LYRAQ_OP_LINEAR_W4A4_LORA = 6
 };
 
-/* Bytes of workspace an operation needs for (m, n, k).  0 for the bare GEMMs (no split-K; the call is kept so that
+/* Bytes of workspace an operation can use for (m, n, k).  0 for the INT8 and FP8 GEMMs (no split-K; the call is kept so that
  * callers written against the reference's getWorkspaceSize, int8_gemm_template.h:683-692, keep working); for the
- * LINEAR_* layer forwards below, the size of the quantized activation plus its scales. */
+ * LINEAR_* layer forwards below, the size of the quantized activation plus its scales.  Where rewriting the operands once makes
+ * the W4A4 GEMM faster (from about a thousand rows on), the W4A4 operations add room for both at one byte per element
+ * (n k + m k + 64 m bytes).  That part is optional: with less (GEMM_W4A4: with none) they run without it and give the same bits. */
 LYRAQ_API size_t lyraq_workspace_bytes(int op, int m, int n, int k);
 
 /* INT8 W8A8: C[m,n] = T( T(float(sum_k A[m,k]*B[n,k]) * (alpha_col[n]*alpha_row)) + bias[n] ).

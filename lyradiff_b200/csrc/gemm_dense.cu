@@ -167,16 +167,6 @@ template<int BLOCK_N, int CTAS> struct GemmSmem {
     static constexpr int kTotal      = kBarOffset + kBarBytes + 1024;   // + alignment slack
 };
 
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, uint32_t smem_src, int x, int y)
-{
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-                 ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_src), "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// all of this thread's committed stores have finished READING shared memory (the box may be overwritten)
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-
 // 32 values of one output row -> global memory, directly (fp32 / int32 outputs, or rows whose pitch rules out TMA).
 template<typename T> __device__ __forceinline__ void store_row32(T* p, int valid, bool vec_ok, const float* v)
 {

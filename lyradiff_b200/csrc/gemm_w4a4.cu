@@ -1,4 +1,4 @@
-// W4A4 GEMM, groups of 64 along K, for sm_100a.
+// W4A4 GEMM, groups of 64 along K, for sm_100a, without scratch memory (gemm_w4a4_wide.cu takes the calls that bring some).
 //
 //   D[m,n] = T( epi( sum_g (float(sum_{k in g} a[m,k]*b[n,k]) * sa[m,g]) * sb[n,g] + bias[n] ) + R[m,n] )
 //
@@ -33,6 +33,7 @@
 // All waits are bounded (see sm100_ptx.cuh); a timeout sets the status word and every role exits.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
+#include "gemm_w4a4.cuh"
 
 namespace lyraq {
 
@@ -65,27 +66,6 @@ constexpr int kScaleSlot   = kSlotGroups * (kBM + kBN) * 4;  // 8 KB: sas[8][128
 constexpr int kScaleOffset = kPStages * kPackedStage + kUStages * kUStage;
 constexpr int kBarOffset   = kScaleOffset + kSSlots * kScaleSlot;
 constexpr int kSmemTotal   = kBarOffset + 512 + 1024;
-
-struct Params {
-    int           M, N, K, G;  // G = K / 64
-    int           m_tiles, n_tiles;
-    const float*  sa;
-    const void*   sb;
-    int           sb_is_f16;
-    int           scale_vec_ok;  // G % 4 == 0 and 16-byte aligned scale arrays: 16-byte scale loads are legal
-    void*         D;
-    int           c_dtype;
-    const void*   bias;
-    const void*   residual;
-    int           gelu;
-    int           round_each;    // round to D's type after every epilogue step (the reference's separate 16-bit kernels)
-    const void*   lora_act;      // [M, 32], fp32 or already of D's 16-bit type, or null
-    int           lora_act_is_f32;
-    const void*   lora_up;       // [N, 32] of D's 16-bit type or null
-    unsigned int* status;
-};
-
-constexpr int kLoraRank = 32;
 
 template<typename T>
 __device__ __forceinline__ void final_store32(const Params& p, const float* acc, int row, int col0, int valid, bool vec_ok)
@@ -700,8 +680,6 @@ extern "C" int lyraq_gemm_w4a4(const uint8_t* A, const uint8_t* B, const float* 
                                const void* residual, int epilogue, int m, int n, int k, void* workspace,
                                size_t workspace_bytes, void* stream)
 {
-    (void)workspace;
-    (void)workspace_bytes;
     if (m == 0 || n == 0) {
         return LYRAQ_OK;
     }
@@ -759,6 +737,10 @@ extern "C" int lyraq_gemm_w4a4(const uint8_t* A, const uint8_t* B, const float* 
     const int sms = device_sm_count();
     if (sms <= 0) {
         return LYRAQ_ERR_CUDA;
+    }
+    if (workspace != nullptr && aligned16(workspace) &&   // lyraq_workspace_bytes asks for it where it pays
+        workspace_bytes >= w4::wide_workspace_bytes((size_t)m, (size_t)n, (size_t)k)) {
+        return w4::launch_wide(p, A, B, workspace, sms, (cudaStream_t)stream);
     }
     CUtensorMap ta, tb;
     int st = make_tmap_bytes_2d(&ta, A, (uint64_t)m, (uint64_t)k / 2, (uint64_t)k / 2, w4::kBM, w4::kPackedRowB, false);

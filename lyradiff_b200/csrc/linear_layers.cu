@@ -2,8 +2,11 @@
 // the quantized activation (and its scales) held in caller-provided workspace.  These are what the reference's layers
 // do around every quantized linear with buffers from their allocator; here the caller owns the buffer.
 #include "common.cuh"
+#include "gemm_w4a4.cuh"
 
 namespace lyraq {
+
+int device_sm_count();  // gemm_dense.cu
 
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -12,6 +15,7 @@ static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; 
 //   LINEAR_INT8 : int8 activation [m, k] | fp32 per-token scales [m]
 //   LINEAR_W4A4 : packed int4 activation [m, k/2] | fp32 group scales [m, k/64]
 //   LINEAR_W4A4_LORA : the same, then the fp32 low-rank activation [m, 32]
+// The W4A4 forwards use what a larger workspace has left for the wide GEMM (gemm_w4a4_wide.cu): w4a4_wide_bytes.
 size_t linear_workspace_bytes(int op, size_t m, size_t k)
 {
     switch (op) {
@@ -24,6 +28,13 @@ size_t linear_workspace_bytes(int op, size_t m, size_t k)
     }
 }
 
+// What the wide W4A4 GEMM would use on top (0 where it is not chosen).  Not required: without it the forward runs the other kernel.
+static size_t w4a4_wide_bytes(int op, size_t m, size_t n, size_t k)
+{
+    const bool w4a4 = op == LYRAQ_OP_GEMM_W4A4 || op == LYRAQ_OP_LINEAR_W4A4 || op == LYRAQ_OP_LINEAR_W4A4_LORA;
+    return w4a4 && n > 0 && (k & 63) == 0 && w4::wide_pays(m, n, k, device_sm_count()) ? w4::wide_workspace_bytes(m, n, k) : 0;
+}
+
 }  // namespace lyraq
 
 using namespace lyraq;
@@ -32,11 +43,10 @@ extern "C" {
 
 size_t lyraq_workspace_bytes(int op, int m, int n, int k)
 {
-    (void)n;
     if (m <= 0 || k <= 0) {
         return 0;
     }
-    return linear_workspace_bytes(op, (size_t)m, (size_t)k);
+    return linear_workspace_bytes(op, (size_t)m, (size_t)k) + w4a4_wide_bytes(op, (size_t)m, n > 0 ? (size_t)n : 0, (size_t)k);
 }
 
 int lyraq_linear_fp8_forward(void* Y, const void* x, int dtype, const float* x_scale, const uint8_t* W, const float* w_scale,
@@ -112,8 +122,10 @@ int lyraq_w4a4_forward(void* D, const void* x, int dtype, const float* smooth, c
     if (st != LYRAQ_OK) {
         return st;
     }
+    const size_t used = linear_workspace_bytes(LYRAQ_OP_LINEAR_W4A4, (size_t)m, (size_t)k);
+    const bool   wide = w4a4_wide_bytes(LYRAQ_OP_LINEAR_W4A4, (size_t)m, (size_t)n, (size_t)k) != 0;
     return lyraq_gemm_w4a4(q, W, qs, w_scale, w_scale_dtype, D, dtype, nullptr, LYRAQ_F32, nullptr, bias, residual, epilogue, m, n, k,
-                           nullptr, 0, stream);
+                           wide ? q + used : nullptr, wide ? workspace_bytes - used : 0, stream);
 }
 
 int lyraq_w4a4_lora_forward(void* D, const void* x, int dtype, const float* smooth, const uint8_t* W, const void* w_scale,
@@ -141,8 +153,10 @@ int lyraq_w4a4_lora_forward(void* D, const void* x, int dtype, const float* smoo
     if (st != LYRAQ_OK) {
         return st;
     }
-    return lyraq_gemm_w4a4(q, W, qs, w_scale, w_scale_dtype, D, dtype, act, LYRAQ_F32, lora_up, bias, residual, epilogue, m, n, k, nullptr,
-                           0, stream);
+    const size_t used = linear_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (size_t)m, (size_t)k);
+    const bool   wide = w4a4_wide_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (size_t)m, (size_t)n, (size_t)k) != 0;
+    return lyraq_gemm_w4a4(q, W, qs, w_scale, w_scale_dtype, D, dtype, act, LYRAQ_F32, lora_up, bias, residual, epilogue, m, n, k,
+                           wide ? q + used : nullptr, wide ? workspace_bytes - used : 0, stream);
 }
 
 }  // extern "C"

@@ -54,6 +54,10 @@ static int static_scratch_ptr(unsigned char** out)
 
 using namespace lyraq;
 
+namespace lyraq {
+size_t linear_workspace_bytes(int op, size_t m, size_t k);  // linear_layers.cu
+}
+
 extern "C" {
 
 // Size of the array; as a side effect resolves its address on the current device (the warm-up described at the top).
@@ -80,8 +84,8 @@ int lyraq_w4a4_forward_static(void* D, const void* x, int dtype, const float* sm
     if (m == 0 || n == 0) {
         return LYRAQ_OK;
     }
-    // the same bytes lyraq_w4a4_forward would ask its caller for; beyond the fixed array the call is refused
-    const size_t need = lyraq_workspace_bytes(LYRAQ_OP_LINEAR_W4A4, m, n, k);
+    // the bytes lyraq_w4a4_forward cannot do without; beyond the fixed array the call is refused
+    const size_t need = (m > 0 && k > 0) ? lyraq::linear_workspace_bytes(LYRAQ_OP_LINEAR_W4A4, (size_t)m, (size_t)k) : 0;
     if (need > kStaticScratchBytes) {
         return LYRAQ_ERR_WORKSPACE;
     }

@@ -151,7 +151,7 @@ Tensor fp8_gemm_gate_residual(const Fp8Weight& w, const Tensor& xq, const Tensor
 // (src/lyradiff/layers/w4a4_gemm_block/W4A4GemmWeight.cc:62-79; the reference's state-dict loader for this layer is
 // empty, so its .bin names serve as keys).
 struct W4Weight {
-    Tensor  packed, w_scale, smooth, lora_down, lora_up, bias, workspace;
+    Tensor  packed, w_scale, smooth, lora_down, lora_up, bias;
     int64_t n = 0, k = 0;
     int     epilogue = LYRAQ_EPI_ROUND_EACH;
 
@@ -177,10 +177,9 @@ struct W4Weight {
     // the whole of W4A4Gemm<T>::forward with the roundings of the 16-bit kernels that follow it in the reference
     Tensor run(const Tensor& x, int64_t m, const Tensor& residual, at::ScalarType dt)
     {
+        // from the allocator for this call only: with the weight's bytes in it, one per linear would double the model
         const size_t need = lyraq_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)n, (int)k);
-        if (!workspace.defined() || (size_t)workspace.numel() < need) {
-            workspace = at::empty({(int64_t)need}, x.options().dtype(at::kByte));
-        }
+        Tensor       workspace = at::empty({(int64_t)need}, x.options().dtype(at::kByte));
         Tensor y = at::empty({m, n}, x.options().dtype(dt));
         check(lyraq_w4a4_lora_forward(y.data_ptr(), x.data_ptr(), dt_code(dt), smooth.data_ptr<float>(), packed.data_ptr<uint8_t>(),
                                       w_scale.data_ptr(), w_scale.scalar_type() == at::kHalf ? LYRAQ_F16 : LYRAQ_F32,

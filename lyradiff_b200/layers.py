@@ -127,7 +127,6 @@ class W4A4Gemm:
         self.lora_down, self.lora_up = lora_down, lora_up
         # round_each: round after every epilogue step (the bits of the reference's GEMM + separate 16-bit kernels)
         self._epi = (ops.EPI_GELU_TANH if gelu else ops.EPI_NONE) | (ops.EPI_ROUND_EACH if round_each else 0)
-        self._ws = None
 
     @classmethod
     def from_float(cls, weight, smooth=None, bias=None, gelu=False, scale_dtype=torch.float16, lora_down=None, lora_up=None):
@@ -138,21 +137,22 @@ class W4A4Gemm:
         return cls(qw, sw, smooth, bias, gelu, lora_down, lora_up)
 
     def forward(self, x, residual=None, out=None):
+        # the workspace comes from the allocator for this call only: it may hold the weight at a byte per element
         m = x.numel() // self.k
         x2 = x.reshape(m, self.k)
         y = out if out is not None else torch.empty(m, self.n, dtype=x.dtype, device=x.device)
         if self.lora_down is not None:
-            self._ws = _workspace(OP_LINEAR_W4A4_LORA, m, self.n, self.k, x.device, self._ws)
+            ws = _workspace(OP_LINEAR_W4A4_LORA, m, self.n, self.k, x.device, None)
             st = _lib.lib().lyraq_w4a4_lora_forward(
                 ops._p(y), ops._p(x2), ops._dt(x2), ops._p(self.smooth), ops._p(self.qweight), ops._p(self.w_scale),
                 ops._dt(self.w_scale), ops._p(self.lora_down), ops._p(self.lora_up), ops._p(self.bias), ops._p(residual),
-                self._epi, m, self.n, self.k, ops._p(self._ws), self._ws.numel(), ops._stream())
+                self._epi, m, self.n, self.k, ops._p(ws), ws.numel(), ops._stream())
             _lib.check(st, "lyraq_w4a4_lora_forward")
             return y.reshape(*x.shape[:-1], self.n)
-        self._ws = _workspace(OP_LINEAR_W4A4, m, self.n, self.k, x.device, self._ws)
+        ws = _workspace(OP_LINEAR_W4A4, m, self.n, self.k, x.device, None)
         st = _lib.lib().lyraq_w4a4_forward(
             ops._p(y), ops._p(x2), ops._dt(x2), ops._p(self.smooth), ops._p(self.qweight), ops._p(self.w_scale),
             ops._dt(self.w_scale), ops._p(self.bias), ops._p(residual), self._epi, m,
-            self.n, self.k, ops._p(self._ws), self._ws.numel(), ops._stream())
+            self.n, self.k, ops._p(ws), ws.numel(), ops._stream())
         _lib.check(st, "lyraq_w4a4_forward")
         return y.reshape(*x.shape[:-1], self.n)

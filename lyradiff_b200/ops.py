@@ -13,6 +13,7 @@ from . import _lib
 F16, BF16, F32, S32, E4M3 = 0, 1, 2, 3, 4
 SCALE_PER_TENSOR, SCALE_PER_TOKEN, SCALE_PER_TOKEN_DYNAMIC = 0, 1, 2
 EPI_NONE, EPI_GELU_TANH, EPI_ROUND_EACH = 0, 1, 2
+OP_GEMM_W4A4 = 2
 
 _DTYPES = {torch.float16: F16, torch.bfloat16: BF16, torch.float32: F32, torch.int32: S32}
 
@@ -317,20 +318,24 @@ def gemm_fp8_quant_out(W, w_scale, X, x_scale, Yq, y_scale, dtype, bias=None, re
 
 
 def invoke_fused_w4a4_gemm_and_lora_up(D, A, B, lora_act, lora_up, sa, sb, bias=None, residual=None, is_gelu=False,
-                                       round_each=False):
+                                       round_each=False, workspace=None):
     """invokeFusedW4A4GemmAndLoraUp (src/lyradiff/kernels/w4a4_gemm/w4a4_gemm.h:19-30) with the bias / GELU / residual
     kernels that follow it fused in.  A uint8 [m,k/2], B uint8 [n,k/2], sa fp32 [m,k/64], sb fp32|fp16 [n,k/64];
     lora_act [m,32] fp32 (as the quantizer wrote it) or already of D's dtype, lora_up [n,32] of D's dtype.
-    round_each: round to D's dtype after every epilogue step, as the reference's separate kernels do."""
+    round_each: round to D's dtype after every epilogue step, as the reference's separate kernels do.
+    workspace: uint8 scratch for this call; None takes what lyraq_workspace_bytes asks for from torch's allocator, an empty tensor
+    runs without any (the same bits, slower for many rows)."""
     m, kh = A.shape
     n = B.shape[0]
     k = kh * 2
+    if workspace is None:
+        workspace = torch.empty(_lib.lib().lyraq_workspace_bytes(OP_GEMM_W4A4, m, n, k), dtype=torch.uint8, device=A.device)
     if B.shape[1] != kh or tuple(D.shape) != (m, n):
         raise ValueError("shape mismatch")
     st = _lib.lib().lyraq_gemm_w4a4(_p(A), _p(B), _p(sa), _p(sb), _dt(sb), _p(D), _dt(D), _p(lora_act),
                                     F32 if lora_act is None else _dt(lora_act), _p(lora_up),
                                     _p(bias), _p(residual),
                                     (EPI_GELU_TANH if is_gelu else EPI_NONE) | (EPI_ROUND_EACH if round_each else 0), m, n, k,
-                                    None, 0, _stream())
+                                    _p(workspace) if workspace.numel() else None, workspace.numel(), _stream())
     _lib.check(st, "lyraq_gemm_w4a4")
     return D

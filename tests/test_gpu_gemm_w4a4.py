@@ -201,6 +201,56 @@ def test_lora_up_added_after_the_groups(ops, m, n, k, dt):
     assert_bit_equal(d2, got, "act already of type T")
 
 
+def _wide_bytes(m, n, k):
+    return sum((b + 255) // 256 * 256 for b in (n * k, m * k, 64 * m))
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 8, 64), (256, 256, 64), (257, 8, 128), (300, 72, 192), (384, 264, 1088), (256, 520, 576), (1000, 250, 512),
+                                   (4099, 1544, 1024)])
+@pytest.mark.parametrize("dt,sb_dtype", [(torch.bfloat16, torch.float16), (torch.float16, torch.float32), (torch.float32, torch.float32)])
+def test_wide_kernel_gives_the_same_bits_as_the_one_without_workspace(ops, m, n, k, dt, sb_dtype):
+    """Row, column and K remainders, one and several scale slots (8 groups), an odd number of groups, unaligned scale rows, more
+    tiles than SMs: with every epilogue, and with and without the low-rank step."""
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    r = lambda *s: torch.rand(*s, generator=g, device="cuda")
+    a = torch.randint(0, 256, (m, k // 2), generator=g, device="cuda", dtype=torch.uint8)
+    b = torch.randint(0, 256, (n, k // 2), generator=g, device="cuda", dtype=torch.uint8)
+    a[0], b[0], b[-1] = 0x88, 0x88, 0x77     # the largest sums a group can have: 64 * 64 and -56 * 64
+    sa, sb = r(m, k // 64) * 0.5 + 0.1, (r(n, k // 64) * 0.01 + 0.001).to(sb_dtype)
+    bias, res = r(n).to(dt), r(m, n).to(dt)
+    act, up = (r(m, 32) - 0.5), (r(n, 32) - 0.5).to(dt)
+    none, ample = (torch.empty(size, dtype=torch.uint8, device="cuda") for size in (0, _wide_bytes(m, n, k)))
+    forms = [dict(), dict(bias=bias, is_gelu=True), dict(bias=bias, residual=res, round_each=True)]
+    for lora in (None, act, act.to(dt)):
+        if lora is not None and dt == torch.float32:
+            continue
+        for kw in forms:
+            want, got = (torch.full((m, n), -1.0, dtype=dt, device="cuda") for _ in range(2))
+            for d, ws in ((want, none), (got, ample)):
+                ops.invoke_fused_w4a4_gemm_and_lora_up(d, a, b, lora, None if lora is None else up, sa, sb, workspace=ws, **kw)
+            check_status()
+            assert_bit_equal(got, want.cpu(), str((sorted(kw), lora is not None)))
+
+
+def test_wide_kernel_workspace_is_optional_and_its_size_is_checked(ops):
+    from lyradiff_b200 import _lib
+    L = _lib.lib()
+    assert L.lyraq_workspace_bytes(ops.OP_GEMM_W4A4, 256, 512, 512) == 0          # two tiles: nothing to gain
+    assert L.lyraq_workspace_bytes(ops.OP_GEMM_W4A4, 4608, 12288, 3072) == _wide_bytes(4608, 12288, 3072)
+    need = _wide_bytes(256, 512, 512)
+    a, b = (torch.randint(0, 256, (r, 256), dtype=torch.uint8, device="cuda") for r in (256, 512))
+    sa, sb = torch.ones(256, 8, device="cuda"), torch.ones(512, 8, device="cuda")
+    out = []
+    for size in (0, need - 1, need):
+        ws = torch.full((size + 256,), 0xA5, dtype=torch.uint8, device="cuda")
+        d = torch.empty(256, 512, device="cuda")
+        ops.invoke_fused_w4a4_gemm_and_lora_up(d, a, b, None, None, sa, sb, workspace=ws[:size])
+        check_status()
+        assert bool((ws[size:] == 0xA5).all())
+        out.append(d.cpu())
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+
+
 def test_lora_pointers_must_come_together(ops):
     from lyradiff_b200 import _lib
     d = torch.empty(128, 128, dtype=torch.bfloat16, device="cuda")
