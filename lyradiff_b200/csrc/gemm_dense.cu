@@ -25,6 +25,7 @@
 // block's abort flag and all roles fall through to the common exit, where tensor memory is freed.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
+#include "gemm_skinny.cuh"
 
 namespace lyraq {
 
@@ -1205,6 +1206,12 @@ static int launch_gemm(const void* A, const void* B, GemmParams p, int sms, cuda
 // forced tile configuration for tests and sweeps: 0 = automatic, else block_n * 10 + ctas (2561, 1281, 2562)
 static int g_forced_tile = 0;
 
+// Whether the few-token kernel (gemm_skinny.cu) takes an FP8 problem: a plain epilogue and up to 16 rows (figures there).
+static bool few_tokens(const GemmParams& p)
+{
+    return p.M <= kSkinnyRows && p.epi.gate == nullptr && p.epi.rope == nullptr && p.epi.out_q_scale == nullptr && p.epi.ldc == p.N;
+}
+
 template<int KIND> static int run_gemm(const void* A, const void* B, GemmParams p, cudaStream_t stream)
 {
     if (p.M < 0 || p.N < 0 || p.K < 0) {
@@ -1233,6 +1240,23 @@ template<int KIND> static int run_gemm(const void* A, const void* B, GemmParams 
     }
     if (p.epi.ldc == 0) {
         p.epi.ldc = p.N;
+    }
+    if (KIND == KIND_F8 && g_forced_tile == 0 && few_tokens(p)) {
+        SkinnyParams q{};
+        q.M        = p.M;
+        q.N        = p.N;
+        q.K        = p.K;
+        q.C        = p.epi.C;
+        q.c_dtype  = p.epi.c_dtype;
+        q.s_x      = p.epi.s_a;
+        q.s_w      = p.epi.s_b;
+        q.alpha    = p.epi.alpha;
+        q.beta     = p.epi.beta;
+        q.bias     = p.epi.bias;
+        q.residual = p.epi.residual;
+        q.gelu     = p.epi.gelu;
+        q.status   = p.status;
+        return launch_gemm_skinny(A, B, q, sms, stream);
     }
     TileChoice t = pick_tile(p.M, p.N, p.K, sms);
     if (g_forced_tile != 0) {

@@ -1,0 +1,302 @@
+// FP8 linear for few tokens: Y[m,n] = T(epi(alpha s_x s_w (X W^T) + beta R + bias)) with so few rows of X that the tiles of
+// gemm_tcgen05_kernel (128 or 256 rows of X, all of K) leave most of the chip idle.
+//
+// What bounds it is the weight: every byte of W is read once (28 MB for a modulation linear of FLUX, 4.3 us of HBM), the
+// arithmetic is negligible.  So the operands change places -- 128 rows of W are the M side of the MMA, the rows of X its
+// N side (16, the rest zero-filled by TMA), which wastes no tensor memory and no loads on absent rows -- and
+// K is split over the CTAs of a cluster until all SMs stream: a CTA owns one 128-row block of W and 1/S of K.  The S partial
+// products meet through distributed shared memory: each CTA of the cluster owns 1/S of the block's token columns, receives
+// the others' partials for them and adds them in rank order, so the result does not depend on timing.
+// Measured with the quantize of X in front (one row unless said): [9216, 3072] 15.1 -> 13.2 us, [18432, 3072] 19.2 -> 13.4, 8 rows
+// of [3072, 12288] 29.7 -> 12.5, 16 rows of [12288, 3072] 19.2 -> 14.2.  The store per partial value is what keeps it to 16 rows
+// (64 rows of [9216, 3072]: 34 us against 13).
+//
+//   warp 0  lane 0: TMA producer (W 128 x 128 B, X NB x 128 B per stage).  Before it waits for the kernels in front of it, it
+//           asks its share of W into L2: the weight stream starts while the previous kernel (usually the quantize of X)
+//           still runs.  A prefetch is not a read: whatever that kernel writes is what the loads behind the wait see.
+//   warp 1  lane 0: MMA issuer; the warp owns tensor memory
+//   warps 2-5: accumulator -> shared memory of the owning CTA -> sum, epilogue, store
+// All waits are bounded; a timeout sets the status word and every role leaves.
+#include "common.cuh"
+#include "sm100_ptx.cuh"
+#include "gemm_skinny.cuh"
+
+namespace lyraq {
+
+using namespace sm100;
+
+int make_tmap_bytes_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k_bytes, uint64_t row_stride_bytes,
+                       uint32_t box_rows, uint32_t box_bytes, bool swizzle128);  // gemm_dense.cu
+
+namespace skinny {
+
+constexpr int kWRows   = 128;
+constexpr int kBlockK  = 128;
+constexpr int kWTile   = kWRows * kBlockK;   // 16 KB
+constexpr int kThreads = 192;
+
+template<int NB> struct Layout {
+    static constexpr int kStages    = 5;   // two CTAs share an SM
+    static constexpr int kStage     = kWTile + NB * kBlockK;
+    static constexpr int kRedOffset = kStages * kStage;
+    static constexpr int kRedBytes  = NB * kWRows * 4;
+    static constexpr int kBarOffset = kRedOffset + kRedBytes;
+    static constexpr int kTotal     = kBarOffset + 256 + 1024;
+    static_assert(kTotal <= 115000, "");
+};
+
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int x, int y)
+{
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
+}
+
+__device__ __forceinline__ void st_cluster_f32(uint32_t cluster_addr, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
+}
+
+template<typename T>
+__device__ __forceinline__ void finish(const SkinnyParams& p, float acc, float scale, int m, int n)
+{
+    const size_t at = (size_t)m * (size_t)p.N + (size_t)n;
+    float        t  = acc * scale;
+    if (p.residual != nullptr) {
+        t = fmaf(p.beta, to_f32(reinterpret_cast<const T*>(p.residual)[at]), t);
+    }
+    if (p.bias != nullptr) {
+        t += to_f32(reinterpret_cast<const T*>(p.bias)[n]);
+    }
+    if (p.gelu) {
+        t = gelu_tanh_f32(t);
+    }
+    reinterpret_cast<T*>(p.C)[at] = from_f32<T>(t);
+}
+
+template<int NB>
+__global__ void __launch_bounds__(kThreads, 2)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const SkinnyParams p)
+{
+    using L = Layout<NB>;
+    constexpr int      kStages   = L::kStages;
+    constexpr uint32_t kTmemCols = NB < 32 ? 32 : NB;
+    constexpr uint32_t kIdesc    = umma_idesc(1u, 0u, kWRows, NB);
+
+    extern __shared__ uint8_t smem_raw[];
+    // the dynamic shared window starts at the same offset in every CTA of the kernel, so the layout is that of the peers too
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t*       gen_base  = smem_raw + (smem_base - smem_u32(smem_raw));
+    const uint32_t bars      = smem_base + L::kBarOffset;
+    auto full_bar  = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (kStages + s); };
+    const uint32_t acc_bar    = bars + 8u * (2 * kStages);
+    uint32_t*      tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + L::kBarOffset + 8 * (2 * kStages + 1));
+    volatile int*  abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int rank = (int)cluster_ctarank();
+    const int tile = (int)blockIdx.x / p.splits;
+    const int n0   = (tile % p.n_tiles) * kWRows;
+    const int m0   = (tile / p.n_tiles) * NB;
+    const int kb0  = (int)((long long)p.num_kb * rank / p.splits);
+    const int kb1  = (int)((long long)p.num_kb * (rank + 1) / p.splits);
+
+    grid_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kStages; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        mbar_init(acc_bar, 1);
+        *abort_flag = 0;
+        fence_barrier_init();
+        for (int kb = kb0; kb < kb1; ++kb) {
+            tma_prefetch_2d(&tmap_w, kb * kBlockK, n0);
+        }
+        prefetch_tensormap(&tmap_x);
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    cluster_sync_all();   // every CTA of the cluster runs before a peer writes to its shared memory
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_wait();
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int      stage = 0, issued = 0;
+            uint32_t phase = 0;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
+                    report_timeout(p.status, 0x4100u | (unsigned)stage);
+                    *abort_flag = 1;
+                    break;
+                }
+                const uint32_t dst = smem_base + stage * L::kStage;
+                mbar_arrive_expect_tx(full_bar(stage), (uint32_t)L::kStage);
+                tma_load_2d(dst, &tmap_w, full_bar(stage), kb * kBlockK, n0);
+                tma_load_2d(dst + kWTile, &tmap_x, full_bar(stage), kb * kBlockK, m0);
+                ++issued;
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+            // no copy may be in flight when the block leaves
+            int      s  = stage;
+            uint32_t ph = phase;
+            for (int i = 0; i < kStages && i < issued; ++i) {
+                if (s == 0) {
+                    s = kStages;
+                    ph ^= 1u;
+                }
+                --s;
+                const uint64_t t0 = global_timer_ns();
+                while (!mbar_try_wait(full_bar(s), ph)) {
+                    if (global_timer_ns() - t0 > kWaitLimitNs) {
+                        report_timeout(p.status, 0x4500u | (unsigned)s);
+                        break;
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int      stage = 0;
+            uint32_t phase = 0;
+            bool     ok    = true;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
+                    report_timeout(p.status, 0x4200u | (unsigned)stage);
+                    *abort_flag = 1;
+                    ok = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                const uint64_t adesc = umma_desc_k_sw128(smem_base + stage * L::kStage);
+                const uint64_t bdesc = umma_desc_k_sw128(smem_base + stage * L::kStage + kWTile);
+#pragma unroll
+                for (int k = 0; k < kBlockK / 32; ++k) {
+                    mma_f8f6f4(tmem_base, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kIdesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                }
+                tc_commit(empty_bar(stage));
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+            if (ok) {
+                tc_commit(acc_bar);
+            }
+        }
+    }
+    // ---- accumulator lane = row of W; the CTA of rank r owns the token columns [r NB / S, (r + 1) NB / S)
+    const int slice = NB / p.splits;
+    const int wrow  = (warp & 3) * 32 + lane;
+    bool      ok    = true;
+    if (warp >= 2) {
+        if (!__all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag))) {
+            if (lane == 0) {
+                report_timeout(p.status, 0x4300u);
+            }
+            *abort_flag = 1;
+            ok = false;
+        }
+        if (ok) {
+            tc_fence_after_sync();
+            const uint32_t t_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+            const uint32_t red    = smem_base + L::kRedOffset;
+#pragma unroll 1
+            for (int c0 = 0; c0 < NB && m0 + c0 < p.M; c0 += 16) {
+                uint32_t v[16];
+                tmem_ld_32x16(t_addr + (uint32_t)c0, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int c = c0 + i;
+                    if (m0 + c < p.M) {
+                        const int      owner = c / slice;
+                        const uint32_t at    = red + (uint32_t)(((rank * slice + c - owner * slice) * kWRows + wrow) * 4);
+                        st_cluster_f32(map_to_cta(at, (uint32_t)owner), __uint_as_float(v[i]));
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before_sync();
+    cluster_sync_all();   // all partials of this CTA's columns have arrived
+    tc_fence_after_sync();
+    if (warp == 1) {
+        tmem_dealloc(tmem_base, kTmemCols);
+    }
+    if (warp >= 2 && ok && n0 + wrow < p.N) {
+        const float* red   = reinterpret_cast<const float*>(gen_base + L::kRedOffset);
+        const float  scale = p.alpha * ld_f32(p.s_x) * ld_f32(p.s_w);
+        for (int c = 0; c < slice; ++c) {
+            const int m = m0 + rank * slice + c;
+            if (m >= p.M) {
+                break;
+            }
+            float acc = red[c * kWRows + wrow];
+            for (int s = 1; s < p.splits; ++s) {
+                acc += red[(s * slice + c) * kWRows + wrow];
+            }
+            if (p.c_dtype == LYRAQ_BF16) {
+                finish<__nv_bfloat16>(p, acc, scale, m, n0 + wrow);
+            } else if (p.c_dtype == LYRAQ_F16) {
+                finish<__half>(p, acc, scale, m, n0 + wrow);
+            } else {
+                finish<float>(p, acc, scale, m, n0 + wrow);
+            }
+        }
+    }
+}
+
+template<int NB> int launch(const void* X, const void* W, SkinnyParams p, cudaStream_t stream)
+{
+    using L = Layout<NB>;
+    CUtensorMap tw, tx;
+    int         st = make_tmap_bytes_2d(&tw, W, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, kWRows, kBlockK, true);
+    if (st != LYRAQ_OK) {
+        return st;
+    }
+    st = make_tmap_bytes_2d(&tx, X, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.K, NB, kBlockK, true);
+    if (st != LYRAQ_OK) {
+        return st;
+    }
+    static bool smem_raised[64] = {};
+    st = raise_dynamic_smem_once(gemm_skinny_kernel<NB>, (int)L::kTotal, smem_raised, "cudaFuncSetAttribute(gemm_skinny_kernel)");
+    if (st != LYRAQ_OK) {
+        return st;
+    }
+    const unsigned m_tiles = (unsigned)((p.M + NB - 1) / NB);
+    return cuda_status(launch_kernel(gemm_skinny_kernel<NB>, (unsigned)p.n_tiles * m_tiles * (unsigned)p.splits, (unsigned)kThreads,
+                                     (size_t)L::kTotal, stream, (unsigned)p.splits, tw, tx, p),
+                       "cudaLaunchKernelEx(gemm_skinny_kernel)");
+}
+
+// CTAs along K: as many (1, 2, 4 or 8) as keep the grid within one wave, with at least four K blocks each.
+static int pick_splits(long tiles, int num_kb, long slots)
+{
+    int s = 1;
+    while (s < 8 && tiles * (2 * s) <= slots && num_kb >= 4 * (2 * s)) {
+        s *= 2;
+    }
+    return s;
+}
+
+}  // namespace skinny
+
+int launch_gemm_skinny(const void* X, const void* W, SkinnyParams p, int sms, cudaStream_t stream)
+{
+    using namespace skinny;
+    p.n_tiles = (p.N + kWRows - 1) / kWRows;
+    p.num_kb  = (p.K + kBlockK - 1) / kBlockK;
+    p.splits  = pick_splits(p.n_tiles, p.num_kb, 2l * sms);
+    return launch<kSkinnyRows>(X, W, p, stream);
+}
+
+}  // namespace lyraq

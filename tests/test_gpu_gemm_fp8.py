@@ -153,3 +153,22 @@ def test_fused_output_quantize(ops, tile, dtype, m, n, k):
         assert bool(((dist <= 1) & (same_sign | zeroish)).all())
         assert float((got != want).float().mean()) <= 0.02
     check_status()
+
+
+@pytest.mark.parametrize("m", [1, 2, 7, 15, 16, 17])
+@pytest.mark.parametrize("n,k", [(8, 16), (130, 272), (128, 1024), (264, 4112), (3072, 6144)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_few_tokens(ops, m, n, k, dtype):
+    """The few-token kernel: row counts up to its width and past it, and around the share of them each CTA of a cluster sums, ragged n and k,
+    one to eight CTAs along k.  An fp32 sum of k products in any order is within k 2^-24 of the sum of their magnitudes; the
+    epilogue adds a few fp32 roundings (GELU's approximate tanh: 2^-10 of its argument's magnitude) and one to the output type."""
+    f = workloads.fp8_linear(m, k, n, seed=m + n + k, with_residual=True)
+    mags = (quant.fp8_dequant(f["qx"]).double().abs() @ quant.fp8_dequant(f["qw"]).double().abs().t()) * float(f["s_x"]) * float(f["s_w"])
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -22}[dtype]
+    for kw in (dict(bias=False), dict(residual=True, beta=0.5, alpha=1.25), dict(gelu=True)):
+        y, want = _run(ops, f, dtype, **kw)
+        terms = 1.25 * mags + f["bias"].double().abs()[None, :] + f["residual"].double().abs() + 1.0
+        bound = eps * want.double().abs() + k * 2.0 ** -24 * terms + 2.0 ** -22 * terms + (2.0 ** -10 * want.double().abs() + 2.0 ** -10 if "gelu" in kw else 0.0)
+        d = (y.cpu().double() - want.double()).abs()
+        assert bool((d <= bound).all()), (kw, float((d / bound).max()))
+    check_status()
