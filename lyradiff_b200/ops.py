@@ -36,7 +36,8 @@ def _p(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    # the handle itself: building torch's Stream object for it takes 3 us, a fifth of the smallest call
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def last_status():
