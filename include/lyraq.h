@@ -94,6 +94,11 @@ LYRAQ_API int lyraq_debug_force_gemm_tile(int code);
  * (0, 0) restores normal operation.  It has no counterpart in the reference, whose kernels have no bounded waits. */
 LYRAQ_API int lyraq_debug_attention_wait_test(int skip_loads, unsigned int wait_limit_ms);
 
+/* The same for the few-row FP8 kernel, whose clusters split K: the CTA of rank stalled_rank in each cluster loads nothing, its wait
+ * runs out after wait_limit_ms, and no CTA of the cluster may store anything, because the sums need every rank's part.
+ * (-1, 0) restores normal operation.  It has no counterpart in the reference. */
+LYRAQ_API int lyraq_debug_skinny_wait_test(int stalled_rank, unsigned int wait_limit_ms);
+
 /* Test / sweep hook for the row kernels (quantize, LayerNorm, AdaLN, GEGLU): the most 16-byte vectors one thread
  * holds (4 or 6, default 6) before a row is given to a team twice as large.  Process-wide, not thread-safe.
  * No counterpart in the reference, whose kernels fix columns-per-thread per supported width

@@ -16,7 +16,8 @@
 //           still runs.  A prefetch is not a read: whatever that kernel writes is what the loads behind the wait see.
 //   warp 1  lane 0: MMA issuer; the warp owns tensor memory
 //   warps 2-5: accumulator -> shared memory of the owning CTA -> sum, epilogue, store
-// All waits are bounded; a timeout sets the status word and every role leaves.
+// All waits are bounded.  A timeout sets the status word and the abort flag of every CTA of the cluster: the sums a CTA stores
+// need the partial products of all of them, so when one gives up none of the cluster stores anything.
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "gemm_skinny.cuh"
@@ -53,6 +54,11 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int x, int
 __device__ __forceinline__ void st_cluster_f32(uint32_t cluster_addr, float v)
 {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
+}
+
+__device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 
 template<typename T>
@@ -100,6 +106,13 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const int m0   = (tile / p.n_tiles) * NB;
     const int kb0  = (int)((long long)p.num_kb * rank / p.splits);
     const int kb1  = (int)((long long)p.num_kb * (rank + 1) / p.splits);
+    // records a wait that ran out and stops the whole cluster; its writes are visible to the peers behind the barrier in front of the sums
+    auto give_up = [&](unsigned code) {
+        report_timeout(p.status, code);
+        for (int r = 0; r < p.splits; ++r) {
+            st_cluster_u32(map_to_cta(smem_u32(const_cast<int*>(abort_flag)), (uint32_t)r), 1u);
+        }
+    };
 
     grid_launch_dependents();
     if (threadIdx.x == 0) {
@@ -129,10 +142,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         if (lane == 0) {
             int      stage = 0, issued = 0;
             uint32_t phase = 0;
-            for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
-                    report_timeout(p.status, 0x4100u | (unsigned)stage);
-                    *abort_flag = 1;
+            for (int kb = kb0; kb < kb1 && rank != p.stalled_rank; ++kb) {
+                if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.wait_limit_ns)) {
+                    give_up(0x4100u | (unsigned)stage);
                     break;
                 }
                 const uint32_t dst = smem_base + stage * L::kStage;
@@ -156,7 +168,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 --s;
                 const uint64_t t0 = global_timer_ns();
                 while (!mbar_try_wait(full_bar(s), ph)) {
-                    if (global_timer_ns() - t0 > kWaitLimitNs) {
+                    if (global_timer_ns() - t0 > p.wait_limit_ns) {
                         report_timeout(p.status, 0x4500u | (unsigned)s);
                         break;
                     }
@@ -169,9 +181,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             uint32_t phase = 0;
             bool     ok    = true;
             for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
-                    report_timeout(p.status, 0x4200u | (unsigned)stage);
-                    *abort_flag = 1;
+                if (!mbar_wait(full_bar(stage), phase, abort_flag, p.wait_limit_ns)) {
+                    give_up(0x4200u | (unsigned)stage);
                     ok = false;
                     break;
                 }
@@ -196,16 +207,12 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // ---- accumulator lane = row of W; the CTA of rank r owns the token columns [r NB / S, (r + 1) NB / S)
     const int slice = NB / p.splits;
     const int wrow  = (warp & 3) * 32 + lane;
-    bool      ok    = true;
     if (warp >= 2) {
-        if (!__all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag))) {
+        if (!__all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag, p.wait_limit_ns))) {
             if (lane == 0) {
-                report_timeout(p.status, 0x4300u);
+                give_up(0x4300u);
             }
-            *abort_flag = 1;
-            ok = false;
-        }
-        if (ok) {
+        } else {
             tc_fence_after_sync();
             const uint32_t t_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
             const uint32_t red    = smem_base + L::kRedOffset;
@@ -232,7 +239,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     if (warp == 1) {
         tmem_dealloc(tmem_base, kTmemCols);
     }
-    if (warp >= 2 && ok && n0 + wrow < p.N) {
+    if (warp >= 2 && *abort_flag == 0 && n0 + wrow < p.N) {
         const float* red   = reinterpret_cast<const float*>(gen_base + L::kRedOffset);
         const float  scale = p.alpha * ld_f32(p.s_x) * ld_f32(p.s_w);
         for (int c = 0; c < slice; ++c) {
@@ -290,13 +297,26 @@ static int pick_splits(long tiles, int num_kb, long slots)
 
 }  // namespace skinny
 
+// Test hook (lyraq_debug_skinny_wait_test)
+static int                g_stalled_rank  = -1;
+static unsigned long long g_wait_limit_ns = kWaitLimitNs;
+
 int launch_gemm_skinny(const void* X, const void* W, SkinnyParams p, int sms, cudaStream_t stream)
 {
     using namespace skinny;
     p.n_tiles = (p.N + kWRows - 1) / kWRows;
     p.num_kb  = (p.K + kBlockK - 1) / kBlockK;
     p.splits  = pick_splits(p.n_tiles, p.num_kb, 2l * sms);
+    p.stalled_rank  = g_stalled_rank;
+    p.wait_limit_ns = g_wait_limit_ns;
     return launch<kSkinnyRows>(X, W, p, stream);
 }
 
 }  // namespace lyraq
+
+extern "C" int lyraq_debug_skinny_wait_test(int stalled_rank, unsigned int wait_limit_ms)
+{
+    lyraq::g_stalled_rank  = stalled_rank;
+    lyraq::g_wait_limit_ns = wait_limit_ms == 0 ? lyraq::sm100::kWaitLimitNs : (unsigned long long)wait_limit_ms * 1000000ull;
+    return LYRAQ_OK;
+}

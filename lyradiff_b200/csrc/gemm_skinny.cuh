@@ -17,6 +17,8 @@ struct SkinnyParams {
     const void*   residual;                   // [M, N] of c_dtype or null
     int           gelu;
     unsigned int* status;
+    unsigned long long wait_limit_ns;         // filled in by launch_gemm_skinny: longest a single wait may last,
+    int           stalled_rank;               // and the rank of each cluster whose producer loads nothing (test hook; -1: none)
 };
 
 constexpr int kSkinnyRows = 16;   // most rows it takes

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import gemm, quant, workloads
-from tests.util import check_status, cu, rel_err
+from tests.util import assert_bit_equal, check_status, cu, rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -172,3 +172,30 @@ def test_few_tokens(ops, m, n, k, dtype):
         d = (y.cpu().double() - want.double()).abs()
         assert bool((d <= bound).all()), (kw, float((d / bound).max()))
     check_status()
+
+
+@pytest.mark.parametrize("m,n,k,stalled", [(16, 264, 4096, 0), (16, 264, 4096, 5), (1, 9216, 3072, 3), (16, 15360, 3072, 1)])
+def test_few_tokens_store_nothing_when_a_cluster_rank_gives_up(ops, m, n, k, stalled):
+    """Eight, four and two CTAs along k (n / 128 tiles on 148 SMs): one of each cluster loads nothing and its wait runs out; the
+    others have whole partial products of their own, but no sum to store."""
+    from lyradiff_b200 import _lib
+    lib = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    qw, qx = (torch.randint(0, 0x78, (r, k), generator=g, dtype=torch.uint8, device="cuda") for r in (n, m))   # no NaN codes
+    scale = torch.full((1,), 0.001, device="cuda")
+    good, out = (torch.full((m, n), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    ops.gemm_with_residual_and_bias_fp8(qw, scale, qx, scale, good)
+    check_status()
+    assert lib.lyraq_debug_skinny_wait_test(stalled, 50) == 0
+    try:
+        ops.gemm_with_residual_and_bias_fp8(qw, scale, qx, scale, out)   # the launch itself succeeds
+        torch.cuda.synchronize()
+        status, detail = ops.last_status()
+    finally:
+        assert lib.lyraq_debug_skinny_wait_test(-1, 0) == 0
+    assert status == 4 and 0x4000 <= detail < 0x5000, (status, hex(detail))
+    assert bool((out == 7.0).all()), "a timed-out cluster must not store results"
+    assert ops.last_status()[0] == 0                                     # reading the status cleared it
+    ops.gemm_with_residual_and_bias_fp8(qw, scale, qx, scale, out)
+    check_status()
+    assert_bit_equal(out, good.cpu(), "after a timed-out launch")
