@@ -19,6 +19,8 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
@@ -239,6 +241,101 @@ inline void cuda_check(cudaError_t e, const char* what)
         throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
     }
 }
+/* Device memory for the length of one call, in stream order, shared by all layers of a device: one call's worth stays reserved
+ * between calls (release threshold), because the default pool gives everything back at each synchronisation and mapping it again
+ * costs 0.5 to 3 ms a call.  The last layer that holds the pool gives it back.  Any number of threads and streams may use it: the
+ * driver hands a block out again only behind the work that was using it. */
+class CallPool {
+public:
+    static std::shared_ptr<CallPool> of_current_device()
+    {
+        static std::mutex              guard;
+        static std::weak_ptr<CallPool> pools[64];
+        int                            device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) {
+            return nullptr;
+        }
+        std::lock_guard<std::mutex> lock(guard);
+        std::shared_ptr<CallPool>   pool = pools[device].lock();
+        if (pool == nullptr) {
+            pool          = std::make_shared<CallPool>(device);
+            pools[device] = pool;
+        }
+        return pool;
+    }
+    explicit CallPool(int device): device_(device)
+    {
+        cudaMemPoolProps props{};
+        props.allocType     = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id   = device;
+        if (cudaMemPoolCreate(&pool_, &props) != cudaSuccess) {
+            pool_ = nullptr;
+            (void)cudaGetLastError();
+        }
+    }
+    CallPool(const CallPool&)            = delete;
+    CallPool& operator=(const CallPool&) = delete;
+    ~CallPool()
+    {
+        if (pool_ != nullptr) {
+            cudaMemPoolDestroy(pool_);  /* blocks still in use by work on a stream are given back behind it */
+        }
+    }
+    int device() const { return device_; }
+    /* null where there is no memory to be had, and while the stream is captured: the allocation would become a node that restricts
+     * what the host may do with its graph */
+    void* take(size_t bytes, cudaStream_t stream)
+    {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        void*                   p       = nullptr;
+        if (pool_ == nullptr) {
+            return nullptr;
+        }
+        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        if (capture != cudaStreamCaptureStatusNone) {
+            return nullptr;
+        }
+        {
+            std::lock_guard<std::mutex> lock(guard_);
+            if (bytes > kept_) {
+                std::uint64_t threshold = bytes + kPoolStep;
+                if (cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &threshold) == cudaSuccess) {
+                    kept_ = bytes;
+                }
+            }
+        }
+        if (cudaMallocFromPoolAsync(&p, bytes, pool_, stream) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        return p;
+    }
+
+private:
+    int           device_;
+    cudaMemPool_t pool_ = nullptr;
+    std::mutex    guard_;
+    size_t        kept_ = 0;
+    static constexpr std::uint64_t kPoolStep = 64u << 20;  /* the driver reserves in steps of 32 MB and counts those */
+};
+
+struct CallScratch {
+    void*        ptr;
+    cudaStream_t stream;
+    CallScratch(CallPool* pool, size_t bytes, cudaStream_t s): ptr(pool != nullptr ? pool->take(bytes, s) : nullptr), stream(s) {}
+    CallScratch(const CallScratch&)            = delete;
+    CallScratch& operator=(const CallScratch&) = delete;
+    ~CallScratch()
+    {
+        if (ptr != nullptr) {
+            cudaFreeAsync(ptr, stream);
+        }
+    }
+};
 template<typename T> inline T from_float(float v);
 template<> inline float from_float<float>(float v) { return v; }
 template<> inline half from_float<half>(float v) { return __float2half(v); }
@@ -374,7 +471,9 @@ private:
 /* W4A4Gemm<T>::forward (src/lyradiff/layers/w4a4_gemm_block/W4A4Gemm.cc:113-169) on raw pointers: int4 quantize + low-rank
  * down projection, grouped GEMM + low-rank up projection -> output [m, d_out] of T, no bias (the reference's layers add it
  * afterwards).  The layer keeps its scratch (quantized input, scales, low-rank activation) between calls and grows it
- * when m grows, as the reference's allocateBuffer does. */
+ * when m grows, as the reference's allocateBuffer does.  The room for both operands at one byte per element, with which the GEMM
+ * is faster for many rows, would be a second copy of every weight if each layer kept it: it is taken for the call only, from a pool
+ * that the layers of a device share, and the call does without where there is none or the stream is captured (the same bits). */
 template<typename T>
 class W4A4Gemm {
 public:
@@ -385,7 +484,7 @@ public:
 
     void forward(T* output, const T* input, size_t m, const W4A4GemmWeight<T>* weights)
     {
-        const size_t need = lyraq_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)d_out_, (int)d_in_);
+        const size_t need = lyraq_workspace_min_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)d_out_, (int)d_in_);
         if (need > workspace_bytes_) {
             cudaFree(workspace_);
             workspace_ = nullptr;
@@ -393,10 +492,17 @@ public:
             lyraq_detail::cuda_check(cudaMalloc(&workspace_, need), "cudaMalloc(W4A4Gemm workspace)");
             workspace_bytes_ = need;
         }
+        const size_t full = lyraq_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)d_out_, (int)d_in_);
+        int device = -1;
+        if (full > need && (pool_ == nullptr || cudaGetDevice(&device) != cudaSuccess || pool_->device() != device)) {
+            pool_ = lyraq_detail::CallPool::of_current_device();
+        }
+        const lyraq_detail::CallScratch scratch(full > need ? pool_.get() : nullptr, full, stream_);
         lyraq_detail::check(lyraq_w4a4_lora_forward(output, input, lyraq_detail::DType<T>::value, weights->smooth,
                                                     reinterpret_cast<const uint8_t*>(weights->packed_weight), weights->weight_scale,
                                                     LYRAQ_F32, weights->lora_down, weights->lora_up, nullptr, nullptr, LYRAQ_EPI_NONE,
-                                                    (int)m, (int)d_out_, (int)d_in_, workspace_, workspace_bytes_, stream_),
+                                                    (int)m, (int)d_out_, (int)d_in_, scratch.ptr ? scratch.ptr : workspace_,
+                                                    scratch.ptr ? full : workspace_bytes_, stream_),
                             "W4A4Gemm::forward");
     }
 
@@ -405,6 +511,7 @@ private:
     cudaStream_t stream_;
     void*        workspace_       = nullptr;
     size_t       workspace_bytes_ = 0;
+    std::shared_ptr<lyraq_detail::CallPool> pool_;
 };
 
 /* The two quantized entry points of cublasMMWrapper (src/lyradiff/utils/cublasMMWrapper.h:300-317 and :354-385),

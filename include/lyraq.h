@@ -222,6 +222,11 @@ enum {
  * (n k + m k + 64 m bytes).  That part is optional: with less (GEMM_W4A4: with none) they run without it and give the same bits. */
 LYRAQ_API size_t lyraq_workspace_bytes(int op, int m, int n, int k);
 
+/* The part of lyraq_workspace_bytes that the operation cannot do without (0 for the bare GEMMs): what a layer may keep between calls.
+ * The rest grows with n k, the weight at one byte per element, and is best taken for the call only.  No counterpart in the
+ * reference, whose layers have one buffer (src/lyradiff/layers/w4a4_gemm_block/W4A4Gemm.cc:21-48). */
+LYRAQ_API size_t lyraq_workspace_min_bytes(int op, int m, int n, int k);
+
 /* INT8 W8A8: C[m,n] = T( T(float(sum_k A[m,k]*B[n,k]) * (alpha_col[n]*alpha_row)) + bias[n] ).
  * A int8 [m,k] row-major, B int8 [n,k] (K contiguous), int32 accumulation (exact), alpha_col fp32 [n],
  * alpha_row fp32 [1] or [m] (row_scale_mode PER_TENSOR / PER_TOKEN), bias of c_dtype [n] or NULL.

@@ -42,6 +42,7 @@ SIGNATURES = {
     "lyraq_geglu_quant_int8": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_size_t, c_size_t,
                                        c_void_p]),
     "lyraq_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "lyraq_workspace_min_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "lyraq_gemm_int8": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int,
                                 c_int, c_void_p, c_size_t, c_void_p]),
     "lyraq_gemm_int8_residual": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p,

@@ -49,6 +49,12 @@ size_t lyraq_workspace_bytes(int op, int m, int n, int k)
     return linear_workspace_bytes(op, (size_t)m, (size_t)k) + w4a4_wide_bytes(op, (size_t)m, n > 0 ? (size_t)n : 0, (size_t)k);
 }
 
+size_t lyraq_workspace_min_bytes(int op, int m, int n, int k)
+{
+    (void)n;
+    return m <= 0 || k <= 0 ? 0 : linear_workspace_bytes(op, (size_t)m, (size_t)k);
+}
+
 int lyraq_linear_fp8_forward(void* Y, const void* x, int dtype, const float* x_scale, const uint8_t* W, const float* w_scale,
                              const void* bias, const void* residual, float beta, int epilogue, int m, int n, int k,
                              void* workspace, size_t workspace_bytes, void* stream)

@@ -4,7 +4,10 @@
 // call site is given) and is exported with plain C types so that a test can drive it through ctypes and compare the
 // result with the same operation issued through the C ABI directly.  A swapped argument in a forwarding template shows
 // up as different bits.  Built by tests/test_gpu_shim.py with g++ against liblyraq.so; no device code here.
+#include <memory>
 #include <string>
+#include <thread>
+#include <vector>
 
 #include "lyradiff_shim.h"
 
@@ -180,5 +183,111 @@ EXPORT int shim_w4a4_layer_from_bins(__nv_bfloat16* out, const __nv_bfloat16* in
         layer.forward(out, in, m, &w);
         layer.forward(out, in, m, &w);  // the kept scratch is reused
         lyraq_detail::cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");  // the weights die with this scope
+    });
+}
+
+static void borrow_weights(W4A4GemmWeight<__nv_bfloat16>& w, const void* packed, const float* w_scale, const float* smooth, const void* down, const void* up)
+{
+    w.packed_weight = (int8_t*)packed;
+    w.weight_scale  = (float*)w_scale;
+    w.smooth        = (float*)smooth;
+    w.lora_down     = (__nv_bfloat16*)down;
+    w.lora_up       = (__nv_bfloat16*)up;
+}
+
+// Device bytes that `count` layers hold once each has run and the stream has been waited for, and that are left when they are gone.
+EXPORT int shim_w4a4_layers_held_bytes(__nv_bfloat16* out, const __nv_bfloat16* in, size_t m, size_t d_out, size_t d_in, const void* packed,
+                                       const float* w_scale, const float* smooth, const void* down, const void* up, int count, cudaStream_t s,
+                                       long long* held, long long* left)
+{
+    return guarded([&] {
+        W4A4GemmWeight<__nv_bfloat16> w;
+        borrow_weights(w, packed, w_scale, smooth, down, up);
+        auto free_bytes = [&] {
+            size_t free = 0, total = 0;
+            lyraq_detail::cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+            lyraq_detail::cuda_check(cudaMemGetInfo(&free, &total), "cudaMemGetInfo");
+            return (long long)free;
+        };
+        W4A4Gemm<__nv_bfloat16>(d_out, d_in, s).forward(out, in, m, &w);   // loads the kernels
+        const long long before = free_bytes();
+        std::vector<std::unique_ptr<W4A4Gemm<__nv_bfloat16>>> layers;
+        for (int i = 0; i < count; ++i) {
+            layers.emplace_back(new W4A4Gemm<__nv_bfloat16>(d_out, d_in, s));
+            layers.back()->forward(out, in, m, &w);
+        }
+        *held = before - free_bytes();
+        layers.clear();
+        *left = before - free_bytes();
+    });
+}
+
+// `threads` host threads, each with a stream and two layers of its own, `rounds` calls apiece; out holds one result per thread.
+EXPORT int shim_w4a4_layers_in_threads(__nv_bfloat16* out, const __nv_bfloat16* in, size_t m, size_t d_out, size_t d_in, const void* packed,
+                                       const float* w_scale, const float* smooth, const void* down, const void* up, int threads, int rounds)
+{
+    return guarded([&] {
+        std::vector<std::string> errors(threads);
+        std::vector<std::thread> pool;
+        for (int t = 0; t < threads; ++t) {
+            pool.emplace_back([=, &errors] {
+                try {
+                    using lyraq_detail::cuda_check;
+                    W4A4GemmWeight<__nv_bfloat16> w;
+                    borrow_weights(w, packed, w_scale, smooth, down, up);
+                    cudaStream_t s;
+                    cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
+                    {
+                        W4A4Gemm<__nv_bfloat16> a(d_out, d_in, s), b(d_out, d_in, s);
+                        for (int i = 0; i < rounds; ++i) {
+                            (i & 1 ? a : b).forward(out + (size_t)t * m * d_out, in, m, &w);
+                            if (i % 3 == 2) {
+                                cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+                            }
+                        }
+                        cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+                    }
+                    cuda_check(cudaStreamDestroy(s), "cudaStreamDestroy");
+                } catch (const std::exception& e) {
+                    errors[t] = e.what();
+                }
+            });
+        }
+        for (auto& t : pool) {
+            t.join();
+        }
+        for (const auto& e : errors) {
+            if (!e.empty()) {
+                throw std::runtime_error(e);
+            }
+        }
+    });
+}
+
+// One layer called once, then captured into a graph that runs twice.
+EXPORT int shim_w4a4_layer_captured(__nv_bfloat16* out, const __nv_bfloat16* in, size_t m, size_t d_out, size_t d_in, const void* packed,
+                                    const float* w_scale, const float* smooth, const void* down, const void* up)
+{
+    return guarded([&] {
+        using lyraq_detail::cuda_check;
+        W4A4GemmWeight<__nv_bfloat16> w;
+        borrow_weights(w, packed, w_scale, smooth, down, up);
+        cudaStream_t s;
+        cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
+        W4A4Gemm<__nv_bfloat16> layer(d_out, d_in, s);
+        layer.forward(out, in, m, &w);
+        cudaGraph_t     graph;
+        cudaGraphExec_t exec;
+        cuda_check(cudaStreamBeginCapture(s, cudaStreamCaptureModeGlobal), "cudaStreamBeginCapture");
+        layer.forward(out, in, m, &w);
+        cuda_check(cudaStreamEndCapture(s, &graph), "cudaStreamEndCapture");
+        cuda_check(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate");
+        cuda_check(cudaMemsetAsync(out, 0, m * d_out * 2, s), "cudaMemsetAsync");
+        cuda_check(cudaGraphLaunch(exec, s), "cudaGraphLaunch");
+        cuda_check(cudaGraphLaunch(exec, s), "cudaGraphLaunch");
+        cuda_check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        cuda_check(cudaGraphExecDestroy(exec), "cudaGraphExecDestroy");
+        cuda_check(cudaGraphDestroy(graph), "cudaGraphDestroy");
+        cuda_check(cudaStreamDestroy(s), "cudaStreamDestroy");
     });
 }

@@ -27,7 +27,7 @@ def _build():
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     libdir = os.path.join(ROOT, "lyradiff_b200")
     cmd = ["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", os.path.join(ROOT, "include"), "-I", os.path.join(cuda, "include"),
-           SRC, "-o", OUT, "-L", libdir, "-llyraq", "-L", os.path.join(cuda, "lib64"), "-lcudart", "-Wl,-rpath," + libdir]
+           SRC, "-o", OUT, "-L", libdir, "-llyraq", "-L", os.path.join(cuda, "lib64"), "-lcudart", "-pthread", "-Wl,-rpath," + libdir]
     r = subprocess.run(cmd, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     return OUT
@@ -256,4 +256,63 @@ def test_flux_w4a4_forms_and_weight_container(shim, ops, tmp_path):
         got = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
         shim("shim_w4a4_layer_from_bins", got, x, m, n, k, prefix.encode(), I(file_type), _stream())
         assert_bit_equal(got, ref.cpu(), "W4A4Gemm::forward from .bin files (type %d)" % file_type)
+    check_status()
+
+
+def _w4a4_tensors(ops, m, n, k):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    r = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    x, down, up = r(m, k).bfloat16(), (r(32, k) * 0.05).bfloat16(), (r(n, 32) * 0.05).bfloat16()
+    smooth = r(k).abs() + 0.5
+    qw, sw = torch.empty(n, k // 2, dtype=torch.uint8, device="cuda"), torch.empty(n, k // 64, device="cuda")
+    ops.weight_quant_int4_g64(qw, sw, (r(n, k) * 0.02).bfloat16())
+    return x, qw, sw, smooth, down, up
+
+
+def test_w4a4_layers_hold_only_their_activation_scratch(shim, ops):
+    """Where the GEMM can use room for the weight at a byte per element, a layer must not keep it: eight layers after a call hold
+    what their quantized activations need (2 MB is the device's allocation step) and one call's room together (and up to 64 MB, two
+    of the pool's steps), and nothing when they are gone."""
+    from lyradiff_b200 import _lib, layers
+    L = _lib.lib()
+    m, k, count = 1024, 3072, 8
+    for n in (9216, 12288):
+        full = L.lyraq_workspace_bytes(layers.OP_LINEAR_W4A4_LORA, m, n, k)
+        assert full > n * k                                                                   # the call can use it
+        need = L.lyraq_workspace_min_bytes(layers.OP_LINEAR_W4A4_LORA, m, n, k)
+        x, qw, sw, smooth, down, up = _w4a4_tensors(ops, m, n, k)
+        got = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        held, left = ctypes.c_longlong(), ctypes.c_longlong()
+        shim("shim_w4a4_layers_held_bytes", got, x, m, n, k, qw, sw, smooth, down, up, I(count), _stream(), ctypes.byref(held), ctypes.byref(left))
+        assert held.value <= count * (need + (2 << 20)) + full + (64 << 20), (n, held.value, need, full)
+        assert left.value <= 0, left.value
+        want = layers.W4A4Gemm(qw, sw, smooth=smooth, lora_down=down, lora_up=up).forward(x)
+        assert_bit_equal(got, want.cpu(), "n = %d" % n)
+        del x, qw, sw, smooth, down, up, got, want
+    check_status()
+
+
+def test_w4a4_layers_of_several_threads_share_the_pool(shim, ops):
+    from lyradiff_b200 import layers
+    m, n, k, threads = 1024, 9216, 3072, 3
+    x, qw, sw, smooth, down, up = _w4a4_tensors(ops, m, n, k)
+    want = layers.W4A4Gemm(qw, sw, smooth=smooth, lora_down=down, lora_up=up).forward(x)
+    got = torch.empty(threads, m, n, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.synchronize()
+    shim("shim_w4a4_layers_in_threads", got, x, m, n, k, qw, sw, smooth, down, up, I(threads), I(12))
+    for t in range(threads):
+        assert_bit_equal(got[t], want.cpu(), "thread %d" % t)
+    check_status()
+
+
+def test_w4a4_layer_runs_under_capture_after_one_call(shim, ops):
+    from lyradiff_b200 import layers
+    m, n, k = 1024, 9216, 3072
+    x, qw, sw, smooth, down, up = _w4a4_tensors(ops, m, n, k)
+    want = layers.W4A4Gemm(qw, sw, smooth=smooth, lora_down=down, lora_up=up).forward(x)
+    got = torch.empty_like(want)
+    torch.cuda.synchronize()
+    shim("shim_w4a4_layer_captured", got, x, m, n, k, qw, sw, smooth, down, up)
+    assert_bit_equal(got, want.cpu(), "captured")
     check_status()
