@@ -6,7 +6,7 @@
 
 namespace lyraq {
 
-int device_sm_count();  // gemm_dense.cu
+constexpr int kB200Sms = 148;
 
 static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -29,10 +29,12 @@ size_t linear_workspace_bytes(int op, size_t m, size_t k)
 }
 
 // What the wide W4A4 GEMM would use on top (0 where it is not chosen).  Not required: without it the forward runs the other kernel.
+// Reckoned for the 148 SMs of a B200 and not for the current device: a size query must leave CUDA alone, or a process that asks
+// before it forks leaves its children without a device.
 static size_t w4a4_wide_bytes(int op, size_t m, size_t n, size_t k)
 {
     const bool w4a4 = op == LYRAQ_OP_GEMM_W4A4 || op == LYRAQ_OP_LINEAR_W4A4 || op == LYRAQ_OP_LINEAR_W4A4_LORA;
-    return w4a4 && n > 0 && (k & 63) == 0 && w4::wide_pays(m, n, k, device_sm_count()) ? w4::wide_workspace_bytes(m, n, k) : 0;
+    return w4a4 && n > 0 && (k & 63) == 0 && w4::wide_pays(m, n, k, kB200Sms) ? w4::wide_workspace_bytes(m, n, k) : 0;
 }
 
 }  // namespace lyraq

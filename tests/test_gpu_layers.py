@@ -1,6 +1,8 @@
 """GPU tests of the quantized-Linear layer forwards (quantize into caller workspace + GEMM in one C-ABI call):
 bit-identical to calling the quantizer and the GEMM separately, and checked against the oracle chain."""
 
+import os
+
 import pytest
 import torch
 
@@ -119,3 +121,33 @@ def test_int8_linear_from_the_reference_bin_layout(layers, tmp_path):
     with pytest.raises(RuntimeError, match="expected 200"):
         layers.SmoothQuantLinear.from_bin(prefix, name, 200, 640)
     check_status()
+
+
+def test_workspace_queries_leave_cuda_alone():
+    """A process may ask for sizes and then fork workers that use the GPU: CUDA cannot be used in a child of a process that has
+    initialised it.  Run apart, because this process has."""
+    import subprocess
+    import sys
+    script = """
+import os, warnings
+warnings.simplefilter("ignore")
+from lyradiff_b200 import _lib
+L = _lib.lib()
+for op in range(7):
+    for m in (1, 1024, 4608):
+        L.lyraq_workspace_bytes(op, m, 12288, 3072)
+        L.lyraq_workspace_min_bytes(op, m, 12288, 3072)
+child = os.fork()
+if child == 0:
+    import torch
+    try:
+        ok = float(torch.ones(4, device="cuda").sum()) == 4.0
+    except RuntimeError as e:
+        print(e)
+        ok = False
+    os._exit(0 if ok else 1)
+raise SystemExit(os.waitstatus_to_exitcode(os.waitpid(child, 0)[1]))
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", script], cwd=root, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
