@@ -178,9 +178,16 @@ struct W4Weight {
     Tensor run(const Tensor& x, int64_t m, const Tensor& residual, at::ScalarType dt)
     {
         // from the allocator for this call only: with the weight's bytes in it, one per linear would double the model
-        const size_t need = lyraq_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)n, (int)k);
-        Tensor       workspace = at::empty({(int64_t)need}, x.options().dtype(at::kByte));
-        Tensor y = at::empty({m, n}, x.options().dtype(dt));
+        size_t     need  = lyraq_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)n, (int)k);
+        const auto bytes = x.options().dtype(at::kByte);
+        Tensor     y     = at::empty({m, n}, x.options().dtype(dt));   // first: the optional bytes must not take its place
+        Tensor     workspace;
+        try {
+            workspace = at::empty({(int64_t)need}, bytes);
+        } catch (const c10::OutOfMemoryError&) {   // the optional part does not fit: the slower kernel, the same bits
+            need      = lyraq_workspace_min_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)n, (int)k);
+            workspace = at::empty({(int64_t)need}, bytes);
+        }
         check(lyraq_w4a4_lora_forward(y.data_ptr(), x.data_ptr(), dt_code(dt), smooth.data_ptr<float>(), packed.data_ptr<uint8_t>(),
                                       w_scale.data_ptr(), w_scale.scalar_type() == at::kHalf ? LYRAQ_F16 : LYRAQ_F32,
                                       lora_down.data_ptr(), lora_up.data_ptr(), ptr(bias), ptr(residual), epilogue, (int)m, (int)n,

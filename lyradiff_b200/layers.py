@@ -142,14 +142,14 @@ class W4A4Gemm:
         x2 = x.reshape(m, self.k)
         y = out if out is not None else torch.empty(m, self.n, dtype=x.dtype, device=x.device)
         if self.lora_down is not None:
-            ws = _workspace(OP_LINEAR_W4A4_LORA, m, self.n, self.k, x.device, None)
+            ws = ops.w4a4_workspace(OP_LINEAR_W4A4_LORA, m, self.n, self.k, x.device)
             st = _lib.lib().lyraq_w4a4_lora_forward(
                 ops._p(y), ops._p(x2), ops._dt(x2), ops._p(self.smooth), ops._p(self.qweight), ops._p(self.w_scale),
                 ops._dt(self.w_scale), ops._p(self.lora_down), ops._p(self.lora_up), ops._p(self.bias), ops._p(residual),
                 self._epi, m, self.n, self.k, ops._p(ws), ws.numel(), ops._stream())
             _lib.check(st, "lyraq_w4a4_lora_forward")
             return y.reshape(*x.shape[:-1], self.n)
-        ws = _workspace(OP_LINEAR_W4A4, m, self.n, self.k, x.device, None)
+        ws = ops.w4a4_workspace(OP_LINEAR_W4A4, m, self.n, self.k, x.device)
         st = _lib.lib().lyraq_w4a4_forward(
             ops._p(y), ops._p(x2), ops._dt(x2), ops._p(self.smooth), ops._p(self.qweight), ops._p(self.w_scale),
             ops._dt(self.w_scale), ops._p(self.bias), ops._p(residual), self._epi, m,

@@ -318,19 +318,29 @@ def gemm_fp8_quant_out(W, w_scale, X, x_scale, Yq, y_scale, dtype, bias=None, re
     return Yq
 
 
+def w4a4_workspace(op, m, n, k, device):
+    """uint8 scratch for one W4A4 call: what lyraq_workspace_bytes asks for, or, where that much is not free, the part that the
+    call cannot do without (the same bits, slower for many rows)."""
+    L = _lib.lib()
+    try:
+        return torch.empty(L.lyraq_workspace_bytes(op, m, n, k), dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return torch.empty(L.lyraq_workspace_min_bytes(op, m, n, k), dtype=torch.uint8, device=device)
+
+
 def invoke_fused_w4a4_gemm_and_lora_up(D, A, B, lora_act, lora_up, sa, sb, bias=None, residual=None, is_gelu=False,
                                        round_each=False, workspace=None):
     """invokeFusedW4A4GemmAndLoraUp (src/lyradiff/kernels/w4a4_gemm/w4a4_gemm.h:19-30) with the bias / GELU / residual
     kernels that follow it fused in.  A uint8 [m,k/2], B uint8 [n,k/2], sa fp32 [m,k/64], sb fp32|fp16 [n,k/64];
     lora_act [m,32] fp32 (as the quantizer wrote it) or already of D's dtype, lora_up [n,32] of D's dtype.
     round_each: round to D's dtype after every epilogue step, as the reference's separate kernels do.
-    workspace: uint8 scratch for this call; None takes what lyraq_workspace_bytes asks for from torch's allocator, an empty tensor
-    runs without any (the same bits, slower for many rows)."""
+    workspace: uint8 scratch for this call; None takes it from torch's allocator (w4a4_workspace), an empty tensor runs without any
+    (the same bits, slower for many rows)."""
     m, kh = A.shape
     n = B.shape[0]
     k = kh * 2
     if workspace is None:
-        workspace = torch.empty(_lib.lib().lyraq_workspace_bytes(OP_GEMM_W4A4, m, n, k), dtype=torch.uint8, device=A.device)
+        workspace = w4a4_workspace(OP_GEMM_W4A4, m, n, k, A.device)
     if B.shape[1] != kh or tuple(D.shape) != (m, n):
         raise ValueError("shape mismatch")
     st = _lib.lib().lyraq_gemm_w4a4(_p(A), _p(B), _p(sa), _p(sb), _dt(sb), _p(D), _dt(D), _p(lora_act),

@@ -151,3 +151,44 @@ raise SystemExit(os.waitstatus_to_exitcode(os.waitpid(child, 0)[1]))
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", script], cwd=root, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.fixture
+def memory_limit():
+    """limit(n): torch's allocator gets n bytes beyond what it holds now."""
+    total = torch.cuda.get_device_properties(0).total_memory
+
+    def limit(extra):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + extra) / total)
+    yield limit
+    torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+@pytest.mark.parametrize("form", ["plain", "lora", "gemm"])
+def test_w4a4_runs_where_the_optional_workspace_does_not_fit(layers, memory_limit, form):
+    """The room that lets the GEMM rewrite its operands (32 MB here) is optional: with 24 MB to be had, enough for the 2 MB that the
+    forward needs in the allocator's 20 MB step, the call runs and gives the same bits."""
+    from lyradiff_b200 import ops
+    m, n, k = 1155, 9216, 3072
+    g = torch.Generator(device="cuda").manual_seed(5)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w = r(m, k), r(n, k)
+    down, up = (r(32, k), r(n, 32)) if form == "lora" else (None, None)
+    lin = layers.W4A4Gemm.from_float(w, lora_down=down, lora_up=up)
+    del w
+    want, got = torch.empty(m, n, dtype=torch.bfloat16, device="cuda"), torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    if form == "gemm":
+        qx, sx = torch.empty(m, k // 2, dtype=torch.uint8, device="cuda"), torch.empty(m, k // 64, device="cuda")
+        ops.invoke_fused_quantize_and_lora_down_simple(None, qx, sx, x, None, torch.ones(k, device="cuda"))
+        call = lambda out: ops.invoke_fused_w4a4_gemm_and_lora_up(out, qx, lin.qweight, None, None, sx, lin.w_scale)
+    else:
+        call = lambda out: lin.forward(x, out=out)
+    call(want)
+    memory_limit(24 << 20)
+    with pytest.raises(torch.OutOfMemoryError):
+        torch.empty(n * k, dtype=torch.uint8, device="cuda")
+    call(got)
+    check_status()
+    assert_bit_equal(got, want.cpu(), form)

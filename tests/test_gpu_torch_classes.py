@@ -248,3 +248,34 @@ def test_densely_launched_forwards_repeat_bit_for_bit(ns):
         bad += int(not (torch.equal(got_i, want_i) and torch.equal(got_t, want_t)))
     check_status()
     assert bad == 0, "%d of 60 forwards differ" % bad
+
+
+def test_int4_block_runs_where_the_optional_workspace_does_not_fit(ns):
+    """The C++ W4A4 linears take room to rewrite their operands where it is free; a block that ran in its own memory still does.
+    The limit is 12 MB below the peak of an unlimited call, whose largest part is that room (24 MB more than the 11 MB needed for
+    the [4608, 4096] -> 1024 linear)."""
+    from tests.test_gpu_flux_block import _int4_state_dict
+    D, heads, head_dim, S = 1024, 8, 128, 4608
+    g = torch.Generator().manual_seed(3)
+    sd = _int4_state_dict("b.", D, 4, head_dim, 7, g)
+    hidden = cu(torch.randn(1, S, D, generator=g).bfloat16())
+    temb = cu(torch.nn.functional.silu(torch.randn(1, D, generator=g)).bfloat16())
+    rope = cu(_rope(1, S, head_dim, g, torch.bfloat16))
+    op = ns.FluxSingleTransformerBlockOp("bf16", D, heads, head_dim, 4, 7)
+    op.initialize(ns.LyraDiffCommonContext())
+    op.reload_model_from_state_dict("b.", sd, "cuda")
+    op.forward(hidden, rope, temb)                        # loads kernels and library handles
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    want = op.forward(hidden, rope, temb)
+    torch.cuda.synchronize()
+    peak = torch.cuda.max_memory_reserved()
+    torch.cuda.empty_cache()
+    try:
+        torch.cuda.set_per_process_memory_fraction((peak - (12 << 20) + want.numel() * 2) / torch.cuda.get_device_properties(0).total_memory)
+        got = op.forward(hidden, rope, temb)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    check_status()
+    assert torch.equal(got, want)
