@@ -99,6 +99,11 @@ LYRAQ_API int lyraq_debug_attention_wait_test(int skip_loads, unsigned int wait_
  * (-1, 0) restores normal operation.  It has no counterpart in the reference. */
 LYRAQ_API int lyraq_debug_skinny_wait_test(int stalled_rank, unsigned int wait_limit_ms);
 
+/* Test / sweep hook: the W4A4 GEMM uses its optional workspace wherever it is given enough (on = 1), not only where that is the faster
+ * way (0, default), so that a test reaches that kernel with small problems.  Process-wide, not thread-safe.  No counterpart in the
+ * reference, which has one W4A4 kernel (src/lyradiff/kernels/w4a4_gemm/w4a4_gemm.cu). */
+LYRAQ_API int lyraq_debug_force_w4a4_wide(int on);
+
 /* Test / sweep hook for the row kernels (quantize, LayerNorm, AdaLN, GEGLU): the most 16-byte vectors one thread
  * holds (4 or 6, default 6) before a row is given to a team twice as large.  Process-wide, not thread-safe.
  * No counterpart in the reference, whose kernels fix columns-per-thread per supported width
@@ -219,7 +224,8 @@ enum {
  * callers written against the reference's getWorkspaceSize, int8_gemm_template.h:683-692, keep working); for the
  * LINEAR_* layer forwards below, the size of the quantized activation plus its scales.  Where rewriting the operands once makes
  * the W4A4 GEMM faster (from about a thousand rows on), the W4A4 operations add room for both at one byte per element
- * (n k + m k + 64 m bytes).  That part is optional: with less (GEMM_W4A4: with none) they run without it and give the same bits. */
+ * (n k + m k + 64 m bytes).  That part is optional: with less (GEMM_W4A4: with none) they run without it and give the same bits, and
+ * more than is asked for changes nothing. */
 LYRAQ_API size_t lyraq_workspace_bytes(int op, int m, int n, int k);
 
 /* The part of lyraq_workspace_bytes that the operation cannot do without (0 for the bare GEMMs): what a layer may keep between calls.

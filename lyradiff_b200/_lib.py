@@ -22,6 +22,7 @@ SIGNATURES = {
     "lyraq_debug_set_dependent_launch": (c_int, [c_int]),
     "lyraq_debug_attention_wait_test": (c_int, [c_int, ctypes.c_uint]),
     "lyraq_debug_skinny_wait_test": (c_int, [c_int, ctypes.c_uint]),
+    "lyraq_debug_force_w4a4_wide": (c_int, [c_int]),
     "lyraq_last_cuda_error": (ctypes.c_char_p, []),
     "lyraq_debug_set_row_vectors_per_thread": (c_int, [c_int]),
     "lyraq_debug_set_special_row_kernels": (c_int, [c_int]),

@@ -1,4 +1,5 @@
-// W4A4 GEMM, groups of 64 along K, for sm_100a, without scratch memory (gemm_w4a4_wide.cu takes the calls that bring some).
+// W4A4 GEMM, groups of 64 along K, for sm_100a, without scratch memory (gemm_w4a4_wide.cu takes the calls that bring some and are
+// faster with it: wide_pays).
 //
 //   D[m,n] = T( epi( sum_g (float(sum_{k in g} a[m,k]*b[n,k]) * sa[m,g]) * sb[n,g] + bias[n] ) + R[m,n] )
 //
@@ -669,11 +670,18 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
 }
 
+static int g_force_wide = 0;   // test hook (lyraq_debug_force_w4a4_wide)
+
 }  // namespace w4
 }  // namespace lyraq
 
 using namespace lyraq;
 
+extern "C" int lyraq_debug_force_w4a4_wide(int on)
+{
+    w4::g_force_wide = on ? 1 : 0;
+    return LYRAQ_OK;
+}
 
 extern "C" int lyraq_gemm_w4a4(const uint8_t* A, const uint8_t* B, const float* sa, const void* sb, int sb_dtype, void* D,
                                int c_dtype, const void* lora_act, int lora_act_dtype, const void* lora_up, const void* bias,
@@ -738,8 +746,9 @@ extern "C" int lyraq_gemm_w4a4(const uint8_t* A, const uint8_t* B, const float* 
     if (sms <= 0) {
         return LYRAQ_ERR_CUDA;
     }
-    if (workspace != nullptr && aligned16(workspace) &&   // lyraq_workspace_bytes asks for it where it pays
-        workspace_bytes >= w4::wide_workspace_bytes((size_t)m, (size_t)n, (size_t)k)) {
+    // a caller may hand every GEMM the arena of its largest: the room alone does not make the wide kernel the faster one
+    if (workspace != nullptr && aligned16(workspace) && workspace_bytes >= w4::wide_workspace_bytes((size_t)m, (size_t)n, (size_t)k) &&
+        (w4::g_force_wide != 0 || w4::wide_pays((size_t)m, (size_t)n, (size_t)k, sms, c_dtype == LYRAQ_F32))) {
         return w4::launch_wide(p, A, B, workspace, sms, (cudaStream_t)stream);
     }
     CUtensorMap ta, tb;

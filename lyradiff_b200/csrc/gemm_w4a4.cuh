@@ -29,16 +29,20 @@ struct Params {
 
 constexpr int kLoraRank = 32;
 
-// Whether the wide path is the faster one.  In units of one wave of gemm_w4a4_kernel's 128 x 128 tiles over all SMs (26.6 us at
-// K = 3072): a wave of the wide kernel's 256 x 128 tiles takes 1.47 (38.5 us measured, not 2), the rewrite of the operands
-// (n + m) k * 1.5 bytes at 5 TB/s and 4 us of launch.  Measured: [4608, 12288, 3072] 24 waves 638 us against 12 waves 489 us;
-// [1024, 12288, 3072] 6 / 3 waves 165 / 137 us; [2048, 3072, 3072] 3 / 2 waves 84 / 89 us.
-inline bool wide_pays(size_t m, size_t n, size_t k, int sms)
+// Whether the wide path is the faster one, in microseconds of each kernel.  A wave of gemm_w4a4_kernel's 128 x 128 tiles over all SMs
+// takes 3.4 + 7.4 (k / 1024), one of the wide kernel's 256 x 128 tiles 7.2 + 10.3 (k / 1024); fp32 rows leave the wide kernel element
+// by element, which adds 26 to a wave.  The rewrite moves 1.5 bytes per element of both operands at 5 TB/s behind a launch of 4.
+// Fitted to 175 measured pairs, m 64 .. 8192, n 3072 .. 21504, k 64 .. 12288: on none of them is the choice more than 2 % slower than
+// the other one.  16-bit outputs: [4608, 12288, 3072] 24 waves 616 us against 12 waves 477; [1024, 12288, 3072] 6 / 3 waves 159 / 137;
+// [2048, 3072, 3072] 3 / 2 waves 84 / 88; [8192, 3072, 512] 11 / 6 waves 80 / 83.  fp32: [4608, 12288, 3072] 655 / 837,
+// [4608, 3072, 12288] 574 / 522.
+inline bool wide_pays(size_t m, size_t n, size_t k, int sms, bool fp32_out)
 {
     const size_t u      = sms > 0 ? (size_t)sms : 148;
     const size_t narrow = ((m + 127) / 128 * ((n + 127) / 128) + u - 1) / u;
     const size_t wide   = ((m + 255) / 256 * ((n + 127) / 128) + u - 1) / u;
-    return 1.47 * (double)wide + 3.5e-5 * (double)(m + n) + 460.0 / (double)k < (double)narrow;
+    const double ki     = (double)k / 1024.0;
+    return (double)wide * (7.2 + 10.3 * ki + (fp32_out ? 26.0 : 0.0)) + 4.0 + 3.1e-4 * (double)(m + n) * ki < (double)narrow * (3.4 + 7.4 * ki);
 }
 
 // Workspace of the wide path: both operands at one byte per element, and the low-rank activation at 16 bits.

@@ -15,7 +15,7 @@ static inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; 
 //   LINEAR_INT8 : int8 activation [m, k] | fp32 per-token scales [m]
 //   LINEAR_W4A4 : packed int4 activation [m, k/2] | fp32 group scales [m, k/64]
 //   LINEAR_W4A4_LORA : the same, then the fp32 low-rank activation [m, 32]
-// The W4A4 forwards use what a larger workspace has left for the wide GEMM (gemm_w4a4_wide.cu): w4a4_wide_bytes.
+// The W4A4 forwards hand what a larger workspace has left to the GEMM, for its wide form (gemm_w4a4_wide.cu): w4a4_wide_bytes.
 size_t linear_workspace_bytes(int op, size_t m, size_t k)
 {
     switch (op) {
@@ -34,7 +34,7 @@ size_t linear_workspace_bytes(int op, size_t m, size_t k)
 static size_t w4a4_wide_bytes(int op, size_t m, size_t n, size_t k)
 {
     const bool w4a4 = op == LYRAQ_OP_GEMM_W4A4 || op == LYRAQ_OP_LINEAR_W4A4 || op == LYRAQ_OP_LINEAR_W4A4_LORA;
-    return w4a4 && n > 0 && (k & 63) == 0 && w4::wide_pays(m, n, k, kB200Sms) ? w4::wide_workspace_bytes(m, n, k) : 0;
+    return w4a4 && n > 0 && (k & 63) == 0 && w4::wide_pays(m, n, k, kB200Sms, false) ? w4::wide_workspace_bytes(m, n, k) : 0;
 }
 
 }  // namespace lyraq
@@ -130,10 +130,9 @@ int lyraq_w4a4_forward(void* D, const void* x, int dtype, const float* smooth, c
     if (st != LYRAQ_OK) {
         return st;
     }
-    const size_t used = linear_workspace_bytes(LYRAQ_OP_LINEAR_W4A4, (size_t)m, (size_t)k);
-    const bool   wide = w4a4_wide_bytes(LYRAQ_OP_LINEAR_W4A4, (size_t)m, (size_t)n, (size_t)k) != 0;
+    const size_t used = linear_workspace_bytes(LYRAQ_OP_LINEAR_W4A4, (size_t)m, (size_t)k);   // the GEMM may use the rest
     return lyraq_gemm_w4a4(q, W, qs, w_scale, w_scale_dtype, D, dtype, nullptr, LYRAQ_F32, nullptr, bias, residual, epilogue, m, n, k,
-                           wide ? q + used : nullptr, wide ? workspace_bytes - used : 0, stream);
+                           q + used, workspace_bytes - used, stream);
 }
 
 int lyraq_w4a4_lora_forward(void* D, const void* x, int dtype, const float* smooth, const uint8_t* W, const void* w_scale,
@@ -161,10 +160,9 @@ int lyraq_w4a4_lora_forward(void* D, const void* x, int dtype, const float* smoo
     if (st != LYRAQ_OK) {
         return st;
     }
-    const size_t used = linear_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (size_t)m, (size_t)k);
-    const bool   wide = w4a4_wide_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (size_t)m, (size_t)n, (size_t)k) != 0;
+    const size_t used = linear_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (size_t)m, (size_t)k);   // the GEMM may use the rest
     return lyraq_gemm_w4a4(q, W, qs, w_scale, w_scale_dtype, D, dtype, act, LYRAQ_F32, lora_up, bias, residual, epilogue, m, n, k,
-                           wide ? q + used : nullptr, wide ? workspace_bytes - used : 0, stream);
+                           q + used, workspace_bytes - used, stream);
 }
 
 }  // extern "C"

@@ -201,6 +201,14 @@ def test_lora_up_added_after_the_groups(ops, m, n, k, dt):
     assert_bit_equal(d2, got, "act already of type T")
 
 
+@pytest.fixture
+def forced_wide():
+    from lyradiff_b200 import _lib
+    assert _lib.lib().lyraq_debug_force_w4a4_wide(1) == 0
+    yield
+    _lib.lib().lyraq_debug_force_w4a4_wide(0)
+
+
 def _wide_bytes(m, n, k):
     return sum((b + 255) // 256 * 256 for b in (n * k, m * k, 64 * m))
 
@@ -208,8 +216,8 @@ def _wide_bytes(m, n, k):
 @pytest.mark.parametrize("m,n,k", [(1, 8, 64), (256, 256, 64), (257, 8, 128), (300, 72, 192), (384, 264, 1088), (256, 520, 576), (1000, 250, 512),
                                    (4099, 1544, 1024)])
 @pytest.mark.parametrize("dt,sb_dtype", [(torch.bfloat16, torch.float16), (torch.float16, torch.float32), (torch.float32, torch.float32)])
-def test_wide_kernel_gives_the_same_bits_as_the_one_without_workspace(ops, m, n, k, dt, sb_dtype):
-    """Row, column and K remainders, one and several scale slots (8 groups), an odd number of groups, unaligned scale rows, more
+def test_wide_kernel_gives_the_same_bits_as_the_one_without_workspace(ops, forced_wide, m, n, k, dt, sb_dtype):
+    """Row, column and K remainders, one and several scale slots (4 groups), an odd number of groups, unaligned scale rows, more
     tiles than SMs: with every epilogue, and with and without the low-rank step."""
     g = torch.Generator(device="cuda").manual_seed(m + n + k)
     r = lambda *s: torch.rand(*s, generator=g, device="cuda")
@@ -226,13 +234,15 @@ def test_wide_kernel_gives_the_same_bits_as_the_one_without_workspace(ops, m, n,
             continue
         for kw in forms:
             want, got = (torch.full((m, n), -1.0, dtype=dt, device="cuda") for _ in range(2))
+            ample.fill_(0xA5)
             for d, ws in ((want, none), (got, ample)):
                 ops.invoke_fused_w4a4_gemm_and_lora_up(d, a, b, lora, None if lora is None else up, sa, sb, workspace=ws, **kw)
             check_status()
             assert_bit_equal(got, want.cpu(), str((sorted(kw), lora is not None)))
+            assert not bool((ample[:n * k] == 0xA5).any())      # it was the wide kernel: no e4m3 code of -8 .. 7 is 0xA5
 
 
-def test_wide_kernel_workspace_is_optional_and_its_size_is_checked(ops):
+def test_wide_kernel_workspace_is_optional_and_its_size_is_checked(ops, forced_wide):
     from lyradiff_b200 import _lib
     L = _lib.lib()
     assert L.lyraq_workspace_bytes(ops.OP_GEMM_W4A4, 256, 512, 512) == 0          # two tiles: nothing to gain
@@ -247,7 +257,55 @@ def test_wide_kernel_workspace_is_optional_and_its_size_is_checked(ops):
         ops.invoke_fused_w4a4_gemm_and_lora_up(d, a, b, None, None, sa, sb, workspace=ws[:size])
         check_status()
         assert bool((ws[size:] == 0xA5).all())
+        assert bool((ws == 0xA5).all()) == (size < need)
         out.append(d.cpu())
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("m,n,k,dt,pays", [(1, 12288, 3072, torch.bfloat16, False), (256, 512, 512, torch.bfloat16, False),
+                                           (2048, 3072, 3072, torch.bfloat16, False), (8192, 3072, 512, torch.float16, False),
+                                           (1024, 3072, 3072, torch.float32, False), (1024, 3072, 3072, torch.bfloat16, True),
+                                           (1024, 3072, 12288, torch.float32, True)])
+def test_wide_kernel_runs_only_where_it_is_the_faster_one(ops, m, n, k, dt, pays):
+    """A workspace of any size leaves the choice to the sizes and the output type: one arena serves every GEMM of a program."""
+    g = torch.Generator(device="cuda").manual_seed(k)
+    a, b = (torch.randint(0, 256, (r, k // 2), generator=g, dtype=torch.uint8, device="cuda") for r in (m, n))
+    sa, sb = torch.rand(m, k // 64, generator=g, device="cuda"), torch.rand(n, k // 64, generator=g, device="cuda")
+    arena = torch.full((_wide_bytes(m, n, k) + (1 << 20),), 0xA5, dtype=torch.uint8, device="cuda")
+    want, got = (torch.empty(m, n, dtype=dt, device="cuda") for _ in range(2))
+    ops.invoke_fused_w4a4_gemm_and_lora_up(want, a, b, None, None, sa, sb, workspace=arena[:0])
+    ops.invoke_fused_w4a4_gemm_and_lora_up(got, a, b, None, None, sa, sb, workspace=arena)
+    check_status()
+    assert_bit_equal(got, want.cpu())
+    assert bool((arena == 0xA5).all()) != pays
+
+
+@pytest.mark.parametrize("lora", [False, True])
+def test_linear_forward_gives_the_gemm_the_rest_of_its_workspace(ops, lora):
+    """The scratch of the quantizer lies in front of the room for the rewritten operands and keeps clear of it: with the required bytes,
+    with all that is asked for, and with one byte less, the same bits; the room is used in the second case only."""
+    from lyradiff_b200 import _lib, layers
+    L = _lib.lib()
+    m, n, k = 1155, 9216, 3072
+    g = torch.Generator(device="cuda").manual_seed(8)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, bias, res, smooth = r(m, k), r(n), r(m, n), torch.rand(k, generator=g, device="cuda") + 0.5
+    down, up = (r(32, k), r(n, 32)) if lora else (None, None)
+    lin = layers.W4A4Gemm.from_float(r(n, k), smooth=smooth, lora_down=down, lora_up=up)
+    op = layers.OP_LINEAR_W4A4_LORA if lora else layers.OP_LINEAR_W4A4
+    need, full = L.lyraq_workspace_min_bytes(op, m, n, k), L.lyraq_workspace_bytes(op, m, n, k)
+    assert full == need + _wide_bytes(m, n, k)
+    out = []
+    for size in (need, full - 1, full):
+        ws = torch.full((full + 256,), 0xA5, dtype=torch.uint8, device="cuda")
+        y = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+        weights = (ops._p(smooth), ops._p(lin.qweight), ops._p(lin.w_scale), ops._dt(lin.w_scale)) + ((ops._p(down), ops._p(up)) if lora else ())
+        forward = L.lyraq_w4a4_lora_forward if lora else L.lyraq_w4a4_forward
+        assert forward(ops._p(y), ops._p(x), ops._dt(x), *weights, ops._p(bias), ops._p(res), ops.EPI_GELU_TANH, m, n, k, ops._p(ws), size,
+                       ops._stream()) == 0
+        check_status()
+        assert bool((ws[need:] == 0xA5).all()) == (size < full) and bool((ws[size:] == 0xA5).all())
+        out.append(y.cpu())
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
 
 
