@@ -174,9 +174,9 @@ def test_few_tokens(ops, m, n, k, dtype):
     check_status()
 
 
-@pytest.mark.parametrize("m,n,k,stalled", [(16, 264, 4096, 0), (16, 264, 4096, 5), (1, 9216, 3072, 3), (16, 15360, 3072, 1)])
+@pytest.mark.parametrize("m,n,k,stalled", [(16, 264, 4096, 0), (16, 264, 4096, 5), (1, 8192, 3072, 3), (16, 15360, 3072, 1)])
 def test_few_tokens_store_nothing_when_a_cluster_rank_gives_up(ops, m, n, k, stalled):
-    """Eight, four and two CTAs along k (n / 128 tiles on 148 SMs): one of each cluster loads nothing and its wait runs out; the
+    """Eight, four and two CTAs along k: one of each cluster loads nothing and its wait runs out; the
     others have whole partial products of their own, but no sum to store."""
     from lyradiff_b200 import _lib
     lib = _lib.lib()
@@ -199,3 +199,20 @@ def test_few_tokens_store_nothing_when_a_cluster_rank_gives_up(ops, m, n, k, sta
     ops.gemm_with_residual_and_bias_fp8(qw, scale, qx, scale, out)
     check_status()
     assert_bit_equal(out, good.cpu(), "after a timed-out launch")
+
+
+@pytest.mark.parametrize("m", [1, 3, 7, 16])
+@pytest.mark.parametrize("n,k", [(264, 4096), (4224, 4096), (4352, 4096), (3072, 3072), (9088, 2048), (9216, 2048), (18944, 1024), (19072, 1024),
+                                 (130, 16)])
+def test_few_tokens_with_every_split_of_k(ops, m, n, k):
+    """One, two, four and eight CTAs along k, and both sides of the tile counts at which fewer are taken (33, 71 and 148 tiles of 128).
+    Operands of 0, 1, -1 and 2 make every partial sum an integer below 2^24, so the fp32 results are exact in any order."""
+    g = torch.Generator(device="cuda").manual_seed(n + m)
+    codes = torch.tensor([0x00, 0x38, 0xB8, 0x40], dtype=torch.uint8, device="cuda")
+    values = torch.tensor([0.0, 1.0, -1.0, 2.0], dtype=torch.float64, device="cuda")
+    iw, ix = (torch.randint(0, 4, (r, k), generator=g, device="cuda") for r in (n, m))
+    one = torch.ones(1, device="cuda")
+    y = torch.empty(m, n, dtype=torch.float32, device="cuda")
+    ops.gemm_with_residual_and_bias_fp8(codes[iw], one, codes[ix], one, y)
+    check_status()
+    assert_bit_equal(y, (values[ix] @ values[iw].t()).float().cpu())
