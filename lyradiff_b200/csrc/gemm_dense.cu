@@ -1206,10 +1206,23 @@ static int launch_gemm(const void* A, const void* B, GemmParams p, int sms, cuda
 // forced tile configuration for tests and sweeps: 0 = automatic, else block_n * 10 + ctas (2561, 1281, 2562)
 static int g_forced_tile = 0;
 
-// Whether the few-token kernel (gemm_skinny.cu) takes an FP8 problem: a plain epilogue and up to 16 rows (figures there).
+// Whether the few-token kernel (gemm_skinny.cu) takes an FP8 problem: a plain epilogue, and so few rows that it is the faster one.
+// Its time grows by 0.1 to 0.25 us a row where the dense kernel's does not grow at all, and what it gains at one row grows with K and,
+// for small K, with the tiles.  Dense against few-token, us: 4 rows of [256, 256] 3.8 / 3.4, 8 rows 3.9 / 4.4, 16 rows 3.9 / 6.2; 6 rows
+// of [12288, 256] 4.9 / 4.4, 10 rows 4.8 / 5.3; 6 rows of [1280, 1024] 5.3 / 5.2, 16 rows 5.3 / 6.3; 12 rows of [3072, 1536] 7.0 / 7.1;
+// 16 rows of [3072, 1664] 7.7 / 7.5 and of [1280, 2048] 6.9 / 5.7.  From 16 K blocks on all 16 rows gain, except that the dense kernel
+// gets 1.4 times faster once X has 128 KB, which with more tiles than four CTAs along K can share is enough for it to win:
+// [12, 12288, 8192] 37.4 / 24.9, [16, 12288, 8192] 23.2 / 25.4.
 static bool few_tokens(const GemmParams& p)
 {
-    return p.M <= kSkinnyRows && p.epi.gate == nullptr && p.epi.rope == nullptr && p.epi.out_q_scale == nullptr && p.epi.ldc == p.N;
+    if (p.M > kSkinnyRows || p.epi.gate != nullptr || p.epi.rope != nullptr || p.epi.out_q_scale != nullptr || p.epi.ldc != p.N) {
+        return false;
+    }
+    const int num_kb = (p.K + 127) / 128, tiles = (p.N + 127) / 128;
+    if (num_kb < 16) {
+        return p.M <= (num_kb < 12 || tiles < 24 ? 4 + num_kb / 4 + (tiles < 96 ? tiles / 32 : 3) : num_kb == 12 ? 12 : 16);
+    }
+    return tiles <= 71 || (long long)p.M * p.K < 128 * 1024;
 }
 
 template<int KIND> static int run_gemm(const void* A, const void* B, GemmParams p, cudaStream_t stream)

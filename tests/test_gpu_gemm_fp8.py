@@ -201,11 +201,11 @@ def test_few_tokens_store_nothing_when_a_cluster_rank_gives_up(ops, m, n, k, sta
     assert_bit_equal(out, good.cpu(), "after a timed-out launch")
 
 
-@pytest.mark.parametrize("m", [1, 3, 7, 16])
+@pytest.mark.parametrize("m", [1, 4, 5, 7, 15, 16])
 @pytest.mark.parametrize("n,k", [(264, 4096), (4224, 4096), (4352, 4096), (3072, 3072), (9088, 2048), (9216, 2048), (18944, 1024), (19072, 1024),
-                                 (130, 16)])
+                                 (130, 16), (256, 256), (4096, 512), (9216, 8192)])
 def test_few_tokens_with_every_split_of_k(ops, m, n, k):
-    """One, two, four and eight CTAs along k, and both sides of the tile counts at which fewer are taken (33, 71 and 148 tiles of 128).
+    """Both sides of the rows at which the dense kernel takes over (small k; 128 KB of X with many tiles).  One, two, four and eight CTAs along k, and both sides of the tile counts at which fewer are taken (33, 71 and 148 tiles of 128).
     Operands of 0, 1, -1 and 2 make every partial sum an integer below 2^24, so the fp32 results are exact in any order."""
     g = torch.Generator(device="cuda").manual_seed(n + m)
     codes = torch.tensor([0x00, 0x38, 0xB8, 0x40], dtype=torch.uint8, device="cuda")
