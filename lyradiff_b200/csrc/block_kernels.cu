@@ -135,10 +135,11 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(T* out, const T* y, 
 }
 
 // w[i] = T(w[i] + T(lora[i] * T(alpha))), each step in T's own arithmetic: loadLora<T>
-// (src/lyradiff/kernels/lora/load_lora.cu:6-14).  n8 vectors of 8 elements, then a scalar tail.  A thread has two vectors of
-// each operand in flight: the kernel is a pass over memory and bound by the bytes outstanding (38.9 -> 37.9 us at
-// [12288, 3072] bf16 = 6.0 TB/s).
-template<typename T>
+// (src/lyradiff/kernels/lora/load_lora.cu:6-14).  n8 vectors of 8 elements, then a scalar tail.  A thread has VECS vectors of
+// each operand in flight: the kernel is a pass over memory and bound by the bytes outstanding, and two do better once every thread
+// has many passes to make (38.4 -> 37.4 us at [12288, 3072] bf16 = 6.0 TB/s, 29.3 -> 28.4 at [9216, 3072]).  With few, one is better:
+// 3.1 against 3.9 us at [1280, 1280], 4.5 against 5.6 at [3072, 1024], 13.9 against 14.3 at [4096, 3072] (five passes).
+template<typename T, int VECS>
 __global__ void __launch_bounds__(256) load_lora_kernel(T* w, const T* lora, size_t n, float alpha)
 {
     using P2 = Pair<T>;
@@ -148,26 +149,27 @@ __global__ void __launch_bounds__(256) load_lora_kernel(T* w, const T* lora, siz
     const size_t   n8     = n >> 3;
     const size_t   stride = (size_t)gridDim.x * blockDim.x;
     const size_t   tid    = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (size_t v0 = tid; v0 < n8; v0 += 2 * stride) {
-        const size_t v1   = v0 + stride;
-        const bool   both = v1 < n8;
-        Vec16        o[2], l[2];
-        o[0] = ld_16(w + (v0 << 3));
-        l[0] = ld_nc_16(lora + (v0 << 3));
-        if (both) {
-            o[1] = ld_16(w + (v1 << 3));
-            l[1] = ld_nc_16(lora + (v1 << 3));
+    for (size_t v0 = tid; v0 < n8; v0 += VECS * stride) {
+        Vec16 o[VECS], l[VECS];
+#pragma unroll
+        for (int q = 0; q < VECS; ++q) {
+            if (q == 0 || v0 + q * stride < n8) {
+                o[q] = ld_16(w + ((v0 + q * stride) << 3));
+                l[q] = ld_nc_16(lora + ((v0 + q * stride) << 3));
+            }
         }
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < VECS; ++q) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 o[q].w[j] = P2::add(o[q].w[j], P2::mul(l[q].w[j], a2));
             }
         }
-        st_16(w + (v0 << 3), o[0]);
-        if (both) {
-            st_16(w + (v1 << 3), o[1]);
+#pragma unroll
+        for (int q = 0; q < VECS; ++q) {
+            if (q == 0 || v0 + q * stride < n8) {
+                st_16(w + ((v0 + q * stride) << 3), o[q]);
+            }
         }
     }
     for (size_t i = (n8 << 3) + tid; i < n; i += stride) {
@@ -298,13 +300,16 @@ int lyraq_load_lora(void* weight, const void* lora, int dtype, float alpha, size
         return LYRAQ_ERR_INVALID_ARG;
     }
     const unsigned grid = stream_grid((n + 7) / 8);
+    const bool     two  = (n >> 3) >= 8ull * 256 * grid;   // eight passes over the grid
     cudaError_t    e;
     if (dtype == LYRAQ_BF16) {
         using T = __nv_bfloat16;
-        e = launch_kernel(load_lora_kernel<T>, grid, 256u, (size_t)0, (cudaStream_t)stream, 1u, (T*)weight, (const T*)lora, n, alpha);
+        e = launch_kernel(two ? load_lora_kernel<T, 2> : load_lora_kernel<T, 1>, grid, 256u, (size_t)0, (cudaStream_t)stream, 1u, (T*)weight,
+                          (const T*)lora, n, alpha);
     } else if (dtype == LYRAQ_F16) {
         using T = __half;
-        e = launch_kernel(load_lora_kernel<T>, grid, 256u, (size_t)0, (cudaStream_t)stream, 1u, (T*)weight, (const T*)lora, n, alpha);
+        e = launch_kernel(two ? load_lora_kernel<T, 2> : load_lora_kernel<T, 1>, grid, 256u, (size_t)0, (cudaStream_t)stream, 1u, (T*)weight,
+                          (const T*)lora, n, alpha);
     } else {
         return LYRAQ_ERR_UNSUPPORTED;
     }

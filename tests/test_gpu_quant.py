@@ -156,9 +156,11 @@ def test_fp8_weight_amax_finds_the_maximum_wherever_it_lies(ops, dtype, n):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("n", [5, 8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 8, 148 * 8 * 256 * 16 + 2043])
+@pytest.mark.parametrize("n", [5, 8, 2048, 148 * 8 * 256 * 8, 148 * 8 * 256 * 8 + 8, 148 * 8 * 256 * 16 + 2043, 148 * 8 * 256 * 64 - 8,
+                               148 * 8 * 256 * 64, 148 * 8 * 256 * 64 + 8, 148 * 8 * 256 * 72 + 2043, 148 * 8 * 256 * 80 + 5])
 def test_load_lora_around_the_two_vector_step(ops, dtype, n):
-    """One and two vectors per thread, the step's remainder and the scalar tail: the bits of the 16-bit operators."""
+    """One and two vectors per thread (two from eight passes over the grid on), each step's remainder and the scalar tail: the bits of
+    the 16-bit operators."""
     g = torch.Generator(device="cuda").manual_seed(n)
     w = torch.randn(n, generator=g, device="cuda").to(dtype)
     lora = torch.randn(n, generator=g, device="cuda").to(dtype)
