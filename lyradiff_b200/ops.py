@@ -35,9 +35,15 @@ def _p(t):
     return t.data_ptr()
 
 
+# torch's call for the bare handle is not one of its public names: a build without it takes the long way round
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
     # the handle itself: building torch's Stream object for it takes 3 us, a fifth of the smallest call
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def last_status():

@@ -106,6 +106,21 @@ def test_unbuilt_quant_levels_are_refused_by_name():
         flux_blocks.FluxSingleTransformerBlockOp()            # the reference's default arguments
 
 
+def test_stream_handle_without_torchs_private_call(monkeypatch):
+    """The handle of the current stream comes from torch's public interface where the private call does not exist."""
+    from lyradiff_b200 import ops
+
+    class Stream:
+        cuda_stream = 1234
+    monkeypatch.setattr(ops, "_raw_stream", None, raising=False)
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: Stream)
+    assert ops._stream() == 1234
+    monkeypatch.setattr(ops, "_raw_stream", lambda device: 5678 + device)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    assert ops._stream() == 5679
+
+
 def test_bench_reference_arm_prints_exactly_one_json_line(tmp_path):
     """What reads bench.py's output takes its standard output as one JSON line: nothing else may be written there (progress
     and libraries' banners go to standard error).  The reference arm runs on the host cores, so this needs no GPU."""
