@@ -1,19 +1,21 @@
 // FP8 linear for few tokens: Y[m,n] = T(epi(alpha s_x s_w (X W^T) + beta R + bias)) with so few rows of X that the tiles of
 // gemm_tcgen05_kernel (128 or 256 rows of X, all of K) leave most of the chip idle.
 //
-// What bounds it is the weight: every byte of W is read once (28 MB for a modulation linear of FLUX, 4.3 us of HBM), the
+// What bounds it is the weight: every byte of W is read once (28 MB for a modulation linear of FLUX, 4.4 us of HBM), the
 // arithmetic is negligible.  So the operands change places -- 128 rows of W are the M side of the MMA, the rows of X its
 // N side (16, the rest zero-filled by TMA), which wastes no tensor memory and no loads on absent rows -- and
 // K is split over the CTAs of a cluster until all SMs stream: a CTA owns one 128-row block of W and 1/S of K.  The S partial
 // products meet through distributed shared memory: each CTA of the cluster owns 1/S of the block's token columns, receives
 // the others' partials for them and adds them in rank order, so the result does not depend on timing.
-// Measured with the quantize of X in front (one row unless said): [9216, 3072] 15.1 -> 13.2 us, [18432, 3072] 19.2 -> 13.4, 8 rows
-// of [3072, 12288] 29.7 -> 12.5, 16 rows of [12288, 3072] 19.2 -> 14.2.  The store per partial value is what keeps it to 16 rows
-// (64 rows of [9216, 3072]: 34 us against 13).
+// Measured with the quantize of X in front, dense kernel -> this one: one row of [9216, 3072] 14.7 -> 9.1 us, of [18432, 3072] 19.3 ->
+// 13.3, 8 rows of [3072, 12288] 29.5 -> 12.0, 16 rows of [12288, 3072] 18.1 -> 14.2.  The store per partial value, 0.1 to 0.25 us a row,
+// is what keeps it to 16 rows, and to fewer for small K (few_tokens in gemm_dense.cu; 64 rows of [9216, 3072]: 34 us against 13).
 //
-//   warp 0  lane 0: TMA producer (W 128 x 128 B, X NB x 128 B per stage).  Before it waits for the kernels in front of it, it
+//   warp 0  lane 0: TMA producer (W 128 x 128 B, X 16 x 128 B per stage).  Before it waits for the kernels in front of it, it
 //           asks its share of W into L2: the weight stream starts while the previous kernel (usually the quantize of X)
-//           still runs.  A prefetch is not a read: whatever that kernel writes is what the loads behind the wait see.
+//           still runs.  A prefetch is not a read: whatever that kernel writes is what the loads behind the wait see.  It asks for the
+//           whole share at once, so of a weight beyond L2's 126 MB some lines may be fetched twice (236 MB of [15360, 15360]: 50 us,
+//           4.7 TB/s; the dense kernel takes 69 for one row).
 //   warp 1  lane 0: MMA issuer; the warp owns tensor memory
 //   warps 2-5: accumulator -> shared memory of the owning CTA -> sum, epilogue, store
 // All waits are bounded.  A timeout sets the status word and the abort flag of every CTA of the cluster: the sums a CTA stores
@@ -36,15 +38,14 @@ constexpr int kBlockK  = 128;
 constexpr int kWTile   = kWRows * kBlockK;   // 16 KB
 constexpr int kThreads = 192;
 
-template<int NB> struct Layout {
-    static constexpr int kStages    = 5;   // two CTAs share an SM
-    static constexpr int kStage     = kWTile + NB * kBlockK;
-    static constexpr int kRedOffset = kStages * kStage;
-    static constexpr int kRedBytes  = NB * kWRows * 4;
-    static constexpr int kBarOffset = kRedOffset + kRedBytes;
-    static constexpr int kTotal     = kBarOffset + 256 + 1024;
-    static_assert(kTotal <= 115000, "");
-};
+constexpr int kRows      = kSkinnyRows;      // N side of the MMA: rows of X, the missing ones zero
+constexpr int kStages    = 5;                // two CTAs share an SM
+constexpr int kStage     = kWTile + kRows * kBlockK;
+constexpr int kRedOffset = kStages * kStage;
+constexpr int kRedBytes  = kRows * kWRows * 4;
+constexpr int kBarOffset = kRedOffset + kRedBytes;
+constexpr int kSmemTotal = kBarOffset + 256 + 1024;
+static_assert(kSmemTotal <= 115000, "");
 
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int x, int y)
 {
@@ -78,32 +79,27 @@ __device__ __forceinline__ void finish(const SkinnyParams& p, float acc, float s
     reinterpret_cast<T*>(p.C)[at] = from_f32<T>(t);
 }
 
-template<int NB>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const SkinnyParams p)
 {
-    using L = Layout<NB>;
-    constexpr int      kStages   = L::kStages;
-    constexpr uint32_t kTmemCols = NB < 32 ? 32 : NB;
-    constexpr uint32_t kIdesc    = umma_idesc(1u, 0u, kWRows, NB);
+    constexpr uint32_t kTmemCols = 32;   // the smallest allocation
+    constexpr uint32_t kIdesc    = umma_idesc(1u, 0u, kWRows, kRows);
 
     extern __shared__ uint8_t smem_raw[];
     // the dynamic shared window starts at the same offset in every CTA of the kernel, so the layout is that of the peers too
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t*       gen_base  = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t bars      = smem_base + L::kBarOffset;
+    const uint32_t bars      = smem_base + kBarOffset;
     auto full_bar  = [&](int s) { return bars + 8u * s; };
     auto empty_bar = [&](int s) { return bars + 8u * (kStages + s); };
     const uint32_t acc_bar    = bars + 8u * (2 * kStages);
-    uint32_t*      tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + L::kBarOffset + 8 * (2 * kStages + 1));
+    uint32_t*      tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + kBarOffset + 8 * (2 * kStages + 1));
     volatile int*  abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank();
-    const int tile = (int)blockIdx.x / p.splits;
-    const int n0   = (tile % p.n_tiles) * kWRows;
-    const int m0   = (tile / p.n_tiles) * NB;
+    const int n0   = (int)blockIdx.x / p.splits * kWRows;
     const int kb0  = (int)((long long)p.num_kb * rank / p.splits);
     const int kb1  = (int)((long long)p.num_kb * (rank + 1) / p.splits);
     // records a wait that ran out and stops the whole cluster; its writes are visible to the peers behind the barrier in front of the sums
@@ -147,10 +143,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                     give_up(0x4100u | (unsigned)stage);
                     break;
                 }
-                const uint32_t dst = smem_base + stage * L::kStage;
-                mbar_arrive_expect_tx(full_bar(stage), (uint32_t)L::kStage);
+                const uint32_t dst = smem_base + stage * kStage;
+                mbar_arrive_expect_tx(full_bar(stage), (uint32_t)kStage);
                 tma_load_2d(dst, &tmap_w, full_bar(stage), kb * kBlockK, n0);
-                tma_load_2d(dst + kWTile, &tmap_x, full_bar(stage), kb * kBlockK, m0);
+                tma_load_2d(dst + kWTile, &tmap_x, full_bar(stage), kb * kBlockK, 0);
                 ++issued;
                 if (++stage == kStages) {
                     stage = 0;
@@ -187,8 +183,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                     break;
                 }
                 tc_fence_after_sync();
-                const uint64_t adesc = umma_desc_k_sw128(smem_base + stage * L::kStage);
-                const uint64_t bdesc = umma_desc_k_sw128(smem_base + stage * L::kStage + kWTile);
+                const uint64_t adesc = umma_desc_k_sw128(smem_base + stage * kStage);
+                const uint64_t bdesc = umma_desc_k_sw128(smem_base + stage * kStage + kWTile);
 #pragma unroll
                 for (int k = 0; k < kBlockK / 32; ++k) {
                     mma_f8f6f4(tmem_base, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), kIdesc, (kb > kb0 || k > 0) ? 1u : 0u);
@@ -205,7 +201,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         }
     }
     // ---- accumulator lane = row of W; the CTA of rank r owns the token columns [r NB / S, (r + 1) NB / S)
-    const int slice = NB / p.splits;
+    const int slice = kRows / p.splits;
     const int wrow  = (warp & 3) * 32 + lane;
     if (warp >= 2) {
         if (!__all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag, p.wait_limit_ns))) {
@@ -214,21 +210,15 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         } else {
             tc_fence_after_sync();
-            const uint32_t t_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-            const uint32_t red    = smem_base + L::kRedOffset;
-#pragma unroll 1
-            for (int c0 = 0; c0 < NB && m0 + c0 < p.M; c0 += 16) {
-                uint32_t v[16];
-                tmem_ld_32x16(t_addr + (uint32_t)c0, v);
-                tmem_ld_wait();
+            uint32_t v[kRows];
+            tmem_ld_32x16(tmem_base + ((uint32_t)((warp & 3) * 32) << 16), v);
+            tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int c = c0 + i;
-                    if (m0 + c < p.M) {
-                        const int      owner = c / slice;
-                        const uint32_t at    = red + (uint32_t)(((rank * slice + c - owner * slice) * kWRows + wrow) * 4);
-                        st_cluster_f32(map_to_cta(at, (uint32_t)owner), __uint_as_float(v[i]));
-                    }
+            for (int c = 0; c < kRows; ++c) {
+                if (c < p.M) {
+                    const int      owner = c / slice;
+                    const uint32_t at    = smem_base + kRedOffset + (uint32_t)(((rank * slice + c - owner * slice) * kWRows + wrow) * 4);
+                    st_cluster_f32(map_to_cta(at, (uint32_t)owner), __uint_as_float(v[c]));
                 }
             }
         }
@@ -240,10 +230,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         tmem_dealloc(tmem_base, kTmemCols);
     }
     if (warp >= 2 && *abort_flag == 0 && n0 + wrow < p.N) {
-        const float* red   = reinterpret_cast<const float*>(gen_base + L::kRedOffset);
+        const float* red   = reinterpret_cast<const float*>(gen_base + kRedOffset);
         const float  scale = p.alpha * ld_f32(p.s_x) * ld_f32(p.s_w);
         for (int c = 0; c < slice; ++c) {
-            const int m = m0 + rank * slice + c;
+            const int m = rank * slice + c;
             if (m >= p.M) {
                 break;
             }
@@ -260,29 +250,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         }
     }
-}
-
-template<int NB> int launch(const void* X, const void* W, SkinnyParams p, cudaStream_t stream)
-{
-    using L = Layout<NB>;
-    CUtensorMap tw, tx;
-    int         st = make_tmap_bytes_2d(&tw, W, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, kWRows, kBlockK, true);
-    if (st != LYRAQ_OK) {
-        return st;
-    }
-    st = make_tmap_bytes_2d(&tx, X, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.K, NB, kBlockK, true);
-    if (st != LYRAQ_OK) {
-        return st;
-    }
-    static bool smem_raised[64] = {};
-    st = raise_dynamic_smem_once(gemm_skinny_kernel<NB>, (int)L::kTotal, smem_raised, "cudaFuncSetAttribute(gemm_skinny_kernel)");
-    if (st != LYRAQ_OK) {
-        return st;
-    }
-    const unsigned m_tiles = (unsigned)((p.M + NB - 1) / NB);
-    return cuda_status(launch_kernel(gemm_skinny_kernel<NB>, (unsigned)p.n_tiles * m_tiles * (unsigned)p.splits, (unsigned)kThreads,
-                                     (size_t)L::kTotal, stream, (unsigned)p.splits, tw, tx, p),
-                       "cudaLaunchKernelEx(gemm_skinny_kernel)");
 }
 
 // Clusters of `size` CTAs that run at once, two CTAs to an SM: a cluster lies within one GPC, and clusters of 4 or 8 leave some of a
@@ -313,12 +280,28 @@ static unsigned long long g_wait_limit_ns = kWaitLimitNs;
 int launch_gemm_skinny(const void* X, const void* W, SkinnyParams p, int sms, cudaStream_t stream)
 {
     using namespace skinny;
-    p.n_tiles = (p.N + kWRows - 1) / kWRows;
-    p.num_kb  = (p.K + kBlockK - 1) / kBlockK;
-    p.splits  = pick_splits(p.n_tiles, p.num_kb, sms);
-    p.stalled_rank  = g_stalled_rank;
-    p.wait_limit_ns = g_wait_limit_ns;
-    return launch<kSkinnyRows>(X, W, p, stream);
+    const int n_tiles = (p.N + kWRows - 1) / kWRows;
+    p.num_kb          = (p.K + kBlockK - 1) / kBlockK;
+    p.splits          = pick_splits(n_tiles, p.num_kb, sms);
+    p.stalled_rank    = g_stalled_rank;
+    p.wait_limit_ns   = g_wait_limit_ns;
+    CUtensorMap tw, tx;
+    int         st = make_tmap_bytes_2d(&tw, W, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, kWRows, kBlockK, true);
+    if (st != LYRAQ_OK) {
+        return st;
+    }
+    st = make_tmap_bytes_2d(&tx, X, (uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.K, kRows, kBlockK, true);
+    if (st != LYRAQ_OK) {
+        return st;
+    }
+    static bool smem_raised[64] = {};
+    st = raise_dynamic_smem_once(gemm_skinny_kernel, kSmemTotal, smem_raised, "cudaFuncSetAttribute(gemm_skinny_kernel)");
+    if (st != LYRAQ_OK) {
+        return st;
+    }
+    return cuda_status(launch_kernel(gemm_skinny_kernel, (unsigned)(n_tiles * p.splits), (unsigned)kThreads, (size_t)kSmemTotal, stream,
+                                     (unsigned)p.splits, tw, tx, p),
+                       "cudaLaunchKernelEx(gemm_skinny_kernel)");
 }
 
 }  // namespace lyraq

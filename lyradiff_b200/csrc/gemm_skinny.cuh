@@ -7,7 +7,7 @@ namespace lyraq {
 
 struct SkinnyParams {
     int           M, N, K;
-    int           n_tiles, num_kb, splits;   // filled in by launch_gemm_skinny
+    int           num_kb, splits;             // filled in by launch_gemm_skinny
     void*         C;                          // [M, N] of c_dtype, F16, BF16 or F32
     int           c_dtype;
     const float*  s_x;

@@ -44,7 +44,6 @@ using namespace sm100;
 int make_tmap_bytes_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k_bytes, uint64_t row_stride_bytes,
                        uint32_t box_rows, uint32_t box_bytes, bool swizzle128);
 int make_tmap_store(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, int elem_bytes, bool wide = false);
-int device_sm_count();
 
 namespace w4 {
 
@@ -150,7 +149,7 @@ constexpr int kBarOffset   = kBiasOffset + kDrainWarps * 128;
 constexpr int kSmemTotal   = kBarOffset + 256 + 1024;
 static_assert(kSmemTotal <= 232448, "");
 constexpr int kCols        = 64;                        // columns of a drain warp
-constexpr int kHalfM       = kBM / 2;                   // rows of an issuer
+constexpr int kHalfM       = kBM / 2;                   // rows of one MMA: an issuer covers a step with two
 // Registers: 384 threads x 168 at launch = 64512; 256 x 216 + 128 x 72 is the same sum.
 constexpr int kDrainRegs   = 216;
 constexpr int kOtherRegs   = 72;
@@ -503,7 +502,7 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             }
         }
     } else {
-        // ------------------------------------------------------------------ drain + epilogue (warps 4 .. 19)
+        // ------------------------------------------------------------------ drain + epilogue (warps 4 .. 11)
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
         const int      quad      = warp & 3;
         const int      part      = (warp - 4) >> 2;     // 64-column half of the tile

@@ -1,8 +1,9 @@
 """Quantized-Linear layers over the C ABI: the host-side mirror of the reference's layer objects for this path.
 
 Each class holds quantized weights and scales the way the reference's *Weight classes do, quantizes on load with the
-device quantizers, owns a workspace for the quantized activation, and its forward() is one C-ABI call
-(lyraq_*_forward).  torch supplies device memory and the stream; nothing is computed in torch.
+device quantizers, and its forward() is one C-ABI call (lyraq_*_forward) with a workspace for the quantized activation, kept between
+calls by the FP8 and INT8 layers and taken per call by W4A4Gemm.  torch supplies device memory and the stream; nothing is computed in
+torch.
 """
 
 import torch
@@ -137,7 +138,7 @@ class W4A4Gemm:
         return cls(qw, sw, smooth, bias, gelu, lora_down, lora_up)
 
     def forward(self, x, residual=None, out=None):
-        # the workspace comes from the allocator for this call only: it may hold the weight at a byte per element
+        # the workspace is for this call only: it may hold the weight at a byte per element
         m = x.numel() // self.k
         x2 = x.reshape(m, self.k)
         y = out if out is not None else torch.empty(m, self.n, dtype=x.dtype, device=x.device)

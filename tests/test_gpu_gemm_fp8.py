@@ -156,11 +156,11 @@ def test_fused_output_quantize(ops, tile, dtype, m, n, k):
 
 
 @pytest.mark.parametrize("m", [1, 2, 7, 15, 16, 17])
-@pytest.mark.parametrize("n,k", [(8, 16), (130, 272), (128, 1024), (264, 4112), (3072, 6144)])
+@pytest.mark.parametrize("n,k", [(8, 16), (130, 272), (128, 1024), (264, 3072), (264, 4112), (3072, 6144)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_few_tokens(ops, m, n, k, dtype):
     """The few-token kernel: row counts up to its width and past it, and around the share of them each CTA of a cluster sums, ragged n and k,
-    one to eight CTAs along k.  An fp32 sum of k products in any order is within k 2^-24 of the sum of their magnitudes; the
+    one, two, four and eight CTAs along k; the larger row counts of the first three shapes, and 17, are the dense kernel's.  An fp32 sum of k products in any order is within k 2^-24 of the sum of their magnitudes; the
     epilogue adds a few fp32 roundings (GELU's approximate tanh: 2^-10 of its argument's magnitude) and one to the output type."""
     f = workloads.fp8_linear(m, k, n, seed=m + n + k, with_residual=True)
     mags = (quant.fp8_dequant(f["qx"]).double().abs() @ quant.fp8_dequant(f["qw"]).double().abs().t()) * float(f["s_x"]) * float(f["s_w"])
