@@ -559,13 +559,13 @@ class FluxBlockInt4(FluxBlock):
     LoRA branch (int4 quantize + LoRA-down, grouped GEMM + LoRA-up + epilogue), proj_out as the reference's two linears."""
     name = "flux_block_int4"
     metric = "flux_single_block_int4_throughput"
-    dtype = "int4 W4A4 linears (s32 per group of 64 in TMEM, f32 across groups) + bf16 library attention"
+    dtype = "int4 W4A4 linears (e4m3 codes of the int4 values, exact sums per group of 64 in TMEM, f32 across groups) + bf16 attention"
 
     def __init__(self, tokens):
         super().__init__(tokens)
         self.workload = self.workload.replace("FP8_W8A8", "INT4_W4A4 (rank-32 LoRA branches)").replace("in FP8 linears", "in W4A4 linears")
         self.launches_per_step = 16
-        self.roof["kernel"] = ("whole block: 4 x (int4 quantize, LoRA-down, gemm_w4a4_kernel) + AdaLN, QK-norm/RoPE, attention and gate "
+        self.roof["kernel"] = ("whole block: 4 x (int4 quantize with LoRA-down, w4_expand_kernel, gemm_w4a4_wide_kernel) + AdaLN, QK-norm/RoPE, attention and gate "
                                "kernels of this library, plus one small library matmul")
 
     def _state_dict(self, g, on_gpu=False):
@@ -722,7 +722,7 @@ class W4A4:
     name = "w4a4"
     metric = "w4a4_g64_linear_throughput"
     unit = "TOP/s"
-    dtype = "s4 expanded to s8 (s32 per group in TMEM, fp32 across groups)"
+    dtype = "s4 rewritten as e4m3 (exact sums per group of 64 in TMEM, fp32 across groups)"
     K, N = 3072, 21504
 
     def __init__(self, tokens):
@@ -731,18 +731,21 @@ class W4A4:
         self.scale = 1e12
         self.workload = ("configs[2]: W4A4 group-64 linear M=%d K=3072 N=21504: int4 per-(token, group) quantize of bf16 X + "
                          "grouped GEMM with fp16 weight group scales -> bf16" % self.tokens)
-        self.launches_per_step = 2
+        self.launches_per_step = 3   # quantize, rewrite of the operands, GEMM
         self.timed_names = ["w4a4_gemm"]
         self.timed_work = [self.work_per_step]
-        self.roof = {"bound": "tensor", "unit": "TOP/s", "kernel": "gemm_w4a4_kernel (1 launch per step)"}
-        # profiles/gemm_w4a4_flux_fused.md: small-case capture scaled by the tiles processed
-        self.traffic = 240.0e6 if self.tokens == 4608 else None
+        self.roof = {"bound": "tensor", "unit": "TOP/s", "kernel": "w4_expand_kernel + gemm_w4a4_wide_kernel (1 launch each per step)"}
+        # profiles/gemm_w4a4_wide_4608x21504.md: both launches
+        self.traffic = 297.6e6 if self.tokens == 4608 else None
 
     def setup_gpu(self, dev):
-        from lyradiff_b200 import ops
+        from lyradiff_b200 import _lib, ops
         self.ops = ops
         g = _gen()
         T, K, N = self.tokens, self.K, self.N
+        if _lib.lib().lyraq_workspace_bytes(ops.OP_GEMM_W4A4, T, N, K) == 0:   # few tokens: the kernel that needs no rewrite
+            self.launches_per_step = 2
+            self.roof["kernel"] = "gemm_w4a4_kernel (1 launch per step)"
         self.x = torch.randn(T, K, generator=g).bfloat16().to(dev)
         w = (torch.randn(N, K, generator=g) * 0.02).bfloat16().to(dev)
         self.qw = torch.empty(N, K // 2, dtype=torch.uint8, device=dev)
