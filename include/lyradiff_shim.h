@@ -241,6 +241,18 @@ inline void cuda_check(cudaError_t e, const char* what)
         throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
     }
 }
+/* Under capture an allocation would become a node that restricts what the host may do with its graph, and creating a pool is not
+ * allowed at all. */
+inline bool capturing(cudaStream_t stream)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return true;   /* the legacy stream while another one is captured */
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 /* Device memory for the length of one call, in stream order, shared by all layers of a device: one call's worth stays reserved
  * between calls (release threshold), because the default pool gives everything back at each synchronisation and mapping it again
  * costs 0.5 to 3 ms a call.  The last layer that holds the pool gives it back.  Any number of threads and streams may use it: the
@@ -283,20 +295,11 @@ public:
         }
     }
     int device() const { return device_; }
-    /* null where there is no memory to be had, and while the stream is captured: the allocation would become a node that restricts
-     * what the host may do with its graph */
+    /* null where there is no memory to be had */
     void* take(size_t bytes, cudaStream_t stream)
     {
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        void*                   p       = nullptr;
+        void* p = nullptr;
         if (pool_ == nullptr) {
-            return nullptr;
-        }
-        if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return nullptr;
-        }
-        if (capture != cudaStreamCaptureStatusNone) {
             return nullptr;
         }
         {
@@ -493,11 +496,12 @@ public:
             workspace_bytes_ = need;
         }
         const size_t full = lyraq_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)d_out_, (int)d_in_);
-        int device = -1;
-        if (full > need && (pool_ == nullptr || cudaGetDevice(&device) != cudaSuccess || pool_->device() != device)) {
+        const bool   optional = full > need && !lyraq_detail::capturing(stream_);
+        int          device   = -1;
+        if (optional && (pool_ == nullptr || cudaGetDevice(&device) != cudaSuccess || pool_->device() != device)) {
             pool_ = lyraq_detail::CallPool::of_current_device();
         }
-        const lyraq_detail::CallScratch scratch(full > need ? pool_.get() : nullptr, full, stream_);
+        const lyraq_detail::CallScratch scratch(optional ? pool_.get() : nullptr, full, stream_);
         lyraq_detail::check(lyraq_w4a4_lora_forward(output, input, lyraq_detail::DType<T>::value, weights->smooth,
                                                     reinterpret_cast<const uint8_t*>(weights->packed_weight), weights->weight_scale,
                                                     LYRAQ_F32, weights->lora_down, weights->lora_up, nullptr, nullptr, LYRAQ_EPI_NONE,

@@ -264,8 +264,8 @@ EXPORT int shim_w4a4_layers_in_threads(__nv_bfloat16* out, const __nv_bfloat16* 
     });
 }
 
-// One layer called once, then captured into a graph that runs twice.
-EXPORT int shim_w4a4_layer_captured(__nv_bfloat16* out, const __nv_bfloat16* in, size_t m, size_t d_out, size_t d_in, const void* packed,
+// One layer called once with first_m rows, then captured with m into a graph that runs twice.
+EXPORT int shim_w4a4_layer_captured(__nv_bfloat16* out, const __nv_bfloat16* in, size_t first_m, size_t m, size_t d_out, size_t d_in, const void* packed,
                                     const float* w_scale, const float* smooth, const void* down, const void* up)
 {
     return guarded([&] {
@@ -275,7 +275,7 @@ EXPORT int shim_w4a4_layer_captured(__nv_bfloat16* out, const __nv_bfloat16* in,
         cudaStream_t s;
         cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
         W4A4Gemm<__nv_bfloat16> layer(d_out, d_in, s);
-        layer.forward(out, in, m, &w);
+        layer.forward(out, in, first_m, &w);
         cudaGraph_t     graph;
         cudaGraphExec_t exec;
         cuda_check(cudaStreamBeginCapture(s, cudaStreamCaptureModeGlobal), "cudaStreamBeginCapture");

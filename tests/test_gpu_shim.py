@@ -306,13 +306,17 @@ def test_w4a4_layers_of_several_threads_share_the_pool(shim, ops):
     check_status()
 
 
-def test_w4a4_layer_runs_under_capture_after_one_call(shim, ops):
-    from lyradiff_b200 import layers
-    m, n, k = 1024, 9216, 3072
-    x, qw, sw, smooth, down, up = _w4a4_tensors(ops, m, n, k)
-    want = layers.W4A4Gemm(qw, sw, smooth=smooth, lora_down=down, lora_up=up).forward(x)
-    got = torch.empty_like(want)
+@pytest.mark.parametrize("first_m,m,n", [(1024, 1024, 9216), (2048, 1024, 3072)])
+def test_w4a4_layer_runs_under_capture_after_one_call(shim, ops, first_m, m, n):
+    """The second case is the layer's first call that could use the optional workspace (1024 rows of 3072 columns can, 2048 cannot)."""
+    from lyradiff_b200 import _lib, layers
+    L, k = _lib.lib(), 3072
+    assert L.lyraq_workspace_bytes(ops.OP_GEMM_W4A4, m, n, k) > 0
+    assert (L.lyraq_workspace_bytes(ops.OP_GEMM_W4A4, first_m, n, k) > 0) == (first_m == m)
+    x, qw, sw, smooth, down, up = _w4a4_tensors(ops, first_m, n, k)
+    want = layers.W4A4Gemm(qw, sw, smooth=smooth, lora_down=down, lora_up=up).forward(x[:m])
+    got = torch.empty(first_m, n, dtype=torch.bfloat16, device="cuda")
     torch.cuda.synchronize()
-    shim("shim_w4a4_layer_captured", got, x, m, n, k, qw, sw, smooth, down, up)
-    assert_bit_equal(got, want.cpu(), "captured")
+    shim("shim_w4a4_layer_captured", got, x, first_m, m, n, k, qw, sw, smooth, down, up)
+    assert_bit_equal(got[:m], want.cpu(), "captured")
     check_status()
