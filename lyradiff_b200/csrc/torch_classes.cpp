@@ -180,13 +180,15 @@ struct W4Weight {
         // from the allocator for this call only: with the weight's bytes in it, one per linear would double the model
         size_t     need  = lyraq_workspace_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)n, (int)k);
         const auto bytes = x.options().dtype(at::kByte);
-        Tensor     y     = at::empty({m, n}, x.options().dtype(dt));   // first: the optional bytes must not take its place
-        Tensor     workspace;
+        Tensor     workspace, y;
         try {
             workspace = at::empty({(int64_t)need}, bytes);
-        } catch (const c10::OutOfMemoryError&) {   // the optional part does not fit: the slower kernel, the same bits
+            y         = at::empty({m, n}, x.options().dtype(dt));
+        } catch (const c10::OutOfMemoryError&) {   // both do not fit: without the optional part, the slower kernel and the same bits
+            workspace = Tensor();
             need      = lyraq_workspace_min_bytes(LYRAQ_OP_LINEAR_W4A4_LORA, (int)m, (int)n, (int)k);
             workspace = at::empty({(int64_t)need}, bytes);
+            y         = at::empty({m, n}, x.options().dtype(dt));
         }
         check(lyraq_w4a4_lora_forward(y.data_ptr(), x.data_ptr(), dt_code(dt), smooth.data_ptr<float>(), packed.data_ptr<uint8_t>(),
                                       w_scale.data_ptr(), w_scale.scalar_type() == at::kHalf ? LYRAQ_F16 : LYRAQ_F32,
