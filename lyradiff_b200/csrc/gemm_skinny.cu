@@ -102,6 +102,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const int n0   = (int)blockIdx.x / p.splits * kWRows;
     const int kb0  = (int)((long long)p.num_kb * rank / p.splits);
     const int kb1  = (int)((long long)p.num_kb * (rank + 1) / p.splits);
+    const uint64_t wait_limit_ns = (uint64_t)p.wait_limit_ms * 1000000u;
     // records a wait that ran out and stops the whole cluster; its writes are visible to the peers behind the barrier in front of the sums
     auto give_up = [&](unsigned code) {
         report_timeout(p.status, code);
@@ -139,7 +140,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             int      stage = 0, issued = 0;
             uint32_t phase = 0;
             for (int kb = kb0; kb < kb1 && rank != p.stalled_rank; ++kb) {
-                if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, p.wait_limit_ns)) {
+                if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, wait_limit_ns)) {
                     give_up(0x4100u | (unsigned)stage);
                     break;
                 }
@@ -164,7 +165,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
                 --s;
                 const uint64_t t0 = global_timer_ns();
                 while (!mbar_try_wait(full_bar(s), ph)) {
-                    if (global_timer_ns() - t0 > p.wait_limit_ns) {
+                    if (global_timer_ns() - t0 > wait_limit_ns) {
                         report_timeout(p.status, 0x4500u | (unsigned)s);
                         break;
                     }
@@ -177,7 +178,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             uint32_t phase = 0;
             bool     ok    = true;
             for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(full_bar(stage), phase, abort_flag, p.wait_limit_ns)) {
+                if (!mbar_wait(full_bar(stage), phase, abort_flag, wait_limit_ns)) {
                     give_up(0x4200u | (unsigned)stage);
                     ok = false;
                     break;
@@ -204,7 +205,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     const int slice = kRows / p.splits;
     const int wrow  = (warp & 3) * 32 + lane;
     if (warp >= 2) {
-        if (!__all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag, p.wait_limit_ns))) {
+        if (!__all_sync(0xffffffffu, mbar_wait(acc_bar, 0u, abort_flag, wait_limit_ns))) {
             if (lane == 0) {
                 give_up(0x4300u);
             }
@@ -274,8 +275,8 @@ static int pick_splits(long tiles, int num_kb, int sms)
 }  // namespace skinny
 
 // Test hook (lyraq_debug_skinny_wait_test)
-static int                g_stalled_rank  = -1;
-static unsigned long long g_wait_limit_ns = kWaitLimitNs;
+static int          g_stalled_rank  = -1;
+static unsigned int g_wait_limit_ms = kWaitLimitNs / 1000000;
 
 int launch_gemm_skinny(const void* X, const void* W, SkinnyParams p, int sms, cudaStream_t stream)
 {
@@ -284,7 +285,7 @@ int launch_gemm_skinny(const void* X, const void* W, SkinnyParams p, int sms, cu
     p.num_kb          = (p.K + kBlockK - 1) / kBlockK;
     p.splits          = pick_splits(n_tiles, p.num_kb, sms);
     p.stalled_rank    = g_stalled_rank;
-    p.wait_limit_ns   = g_wait_limit_ns;
+    p.wait_limit_ms   = g_wait_limit_ms;
     CUtensorMap tw, tx;
     int         st = make_tmap_bytes_2d(&tw, W, (uint64_t)p.N, (uint64_t)p.K, (uint64_t)p.K, kWRows, kBlockK, true);
     if (st != LYRAQ_OK) {
@@ -309,6 +310,6 @@ int launch_gemm_skinny(const void* X, const void* W, SkinnyParams p, int sms, cu
 extern "C" int lyraq_debug_skinny_wait_test(int stalled_rank, unsigned int wait_limit_ms)
 {
     lyraq::g_stalled_rank  = stalled_rank;
-    lyraq::g_wait_limit_ns = wait_limit_ms == 0 ? lyraq::sm100::kWaitLimitNs : (unsigned long long)wait_limit_ms * 1000000ull;
+    lyraq::g_wait_limit_ms = wait_limit_ms == 0 ? (unsigned int)(lyraq::sm100::kWaitLimitNs / 1000000) : wait_limit_ms;
     return LYRAQ_OK;
 }

@@ -6,19 +6,19 @@
 namespace lyraq {
 
 struct SkinnyParams {
-    int           M, N, K;
-    int           num_kb, splits;             // filled in by launch_gemm_skinny
-    void*         C;                          // [M, N] of c_dtype, F16, BF16 or F32
-    int           c_dtype;
+    void*         C;                  // [M, N] of c_dtype, F16, BF16 or F32
     const float*  s_x;
     const float*  s_w;
-    float         alpha, beta;
-    const void*   bias;                       // [N] of c_dtype or null
-    const void*   residual;                   // [M, N] of c_dtype or null
-    int           gelu;
+    const void*   bias;               // [N] of c_dtype or null
+    const void*   residual;           // [M, N] of c_dtype or null
     unsigned int* status;
-    unsigned long long wait_limit_ns;         // filled in by launch_gemm_skinny: longest a single wait may last,
-    int           stalled_rank;               // and the rank of each cluster whose producer loads nothing (test hook; -1: none)
+    int           M, N, K;
+    int           c_dtype;
+    float         alpha, beta;
+    int           gelu;
+    int           num_kb, splits;     // filled in by launch_gemm_skinny, as are
+    int           stalled_rank;       // the rank of each cluster whose producer loads nothing (test hook; -1: none)
+    unsigned int  wait_limit_ms;      // and the longest a single wait may last
 };
 
 constexpr int kSkinnyRows = 16;   // most rows it takes
