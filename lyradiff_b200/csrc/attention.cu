@@ -117,7 +117,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const Params 
     uint32_t*     tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + kBarOffset + 8 * (13 + 2 * kSlots));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     grid_launch_dependents();
@@ -160,7 +160,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const Params 
 
     if (warp == kProducerWarp) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0 && p.skip_loads == 0) {
+        if (p.skip_loads == 0 && elect_one()) {
             mbar_arrive_expect_tx(q_full, (uint32_t)(kQTiles * kTileBytes));
             for (int t = 0; t < kQTiles; ++t) {
                 for (int half = 0; half < 2; ++half) {
@@ -214,7 +214,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const Params 
         }
     } else if (warp >= kMmaWarp) {
         // ------------------------------------------------------------------ MMA issuer of query tile t
-        if (lane == 0) {
+        if (elect_one()) {
             const int      t      = warp - kMmaWarp;
             const uint32_t tcol   = tmem_base + (uint32_t)(t * kTileCols);
             constexpr uint32_t kAb = TypeTag<T>::value == LYRAQ_BF16 ? 1u : 0u;

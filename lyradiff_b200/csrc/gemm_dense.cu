@@ -362,7 +362,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint32_t*      tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + S::kBarOffset + 8 * (2 * kStages + 4));
     volatile int*  abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int      warp    = threadIdx.x >> 5;
+    const int      warp    = warp_index();
     const int      lane    = threadIdx.x & 31;
     const uint32_t rank    = (CTAS == 2) ? cluster_ctarank() : 0u;  // position in the pair; 0 = leader
     const bool     leader  = (rank == 0);
@@ -407,7 +407,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const int num_tiles = p.m_tiles * p.n_tiles;
     const int num_kb    = (p.K + kBlockK - 1) / kBlockK;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ------------------------------------------------------------------ TMA producer (every CTA loads its own halves)
         int      stage = 0;
         uint32_t phase = 0;
@@ -477,7 +477,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 }
             }
         }
-    } else if (warp == 1 && lane == 0 && leader) {
+    } else if (warp == 1 && leader && elect_one()) {
         // ------------------------------------------------------------------ MMA issuer (the leader CTA only)
         int      stage = 0;
         uint32_t phase = 0;

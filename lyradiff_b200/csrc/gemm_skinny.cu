@@ -96,7 +96,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     uint32_t*      tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + kBarOffset + 8 * (2 * kStages + 1));
     volatile int*  abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
     const int rank = (int)cluster_ctarank();
     const int n0   = (int)blockIdx.x / p.splits * kWRows;
@@ -136,7 +136,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     grid_dependency_wait();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int      stage = 0, issued = 0;
             uint32_t phase = 0;
             for (int kb = kb0; kb < kb1 && rank != p.stalled_rank; ++kb) {
@@ -173,7 +173,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int      stage = 0;
             uint32_t phase = 0;
             bool     ok    = true;

@@ -177,7 +177,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint32_t*     tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + kBarOffset + 8 * kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     grid_launch_dependents();
@@ -218,7 +218,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const int num_slots = (num_kb + 3) / 4;  // scale slots per tile
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // -------------------------------------------------------------- TMA producer
             int      stage = 0, issued = 0;
             uint32_t phase = 0;
@@ -264,7 +264,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // -------------------------------------------------------------- MMA issuer
             // One hand-off per K block, not per group: both groups of a block go into the two partial buffers of a pair
             // (pairs alternate between blocks) behind one commit, and the drain warps wait once for both.  A hand-off through

@@ -218,7 +218,7 @@ __device__ __forceinline__ void store_rows16(const Params& p, const float2* acc,
     }
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) {
+    if (elect_one()) {
         tma_store_2d(tmap_d, smem_u32(box), col0, row0);   // clips rows and columns past the end
         tma_store_commit();
     }
@@ -279,7 +279,7 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     uint32_t*     tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + kBarOffset + 8 * kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     grid_launch_dependents();
@@ -319,7 +319,7 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
         if (warp == 0) {
-            if (lane == 0) {
+            if (elect_one()) {
                 // ---------------------------------------------------------- TMA producer
                 int      stage = 0, issued = 0;
                 uint32_t phase = 0;
@@ -365,7 +365,7 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 }
             }
         } else if (warp != 2) {
-            if (lane == 0) {
+            if (elect_one()) {
                 // ---------------------------------------------------------- MMA issuer of the steps n with n & 1 == q
                 const uint32_t q     = (uint32_t)(warp >> 1);
                 const uint32_t d     = tmem_base + q * kBN;
@@ -654,7 +654,7 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             }
             uint16_t* bias_s = reinterpret_cast<uint16_t*>(gen_base + kBiasOffset + (warp - 4) * 128);
             reinterpret_cast<uint32_t*>(bias_s)[lane] = bias2;
-            if (lane == 0) {
+            if (elect_one()) {
                 tma_store_wait_read();   // the last tile's stores have drained the boxes
             }
             __syncwarp();
@@ -684,7 +684,7 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 }
             }
         }
-        if (lane == 0) {
+        if (elect_one()) {
             tma_store_wait_read();  // shared memory must outlive the last stores' reads of it
         }
     }

@@ -69,7 +69,7 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     uint32_t*      tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + kBarOffset + 8 * (2 * kStages + 1));
     volatile int*  abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     grid_launch_dependents();
@@ -98,7 +98,7 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const int row0   = blockIdx.x * kRows;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int      stage = 0, issued = 0;
             uint32_t phase = 0;
             for (int kb = 0; kb < num_kb; ++kb) {
@@ -196,7 +196,7 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 }
             }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         int      stage = 0;
         uint32_t phase = 0;
         bool     ok    = true;
