@@ -130,6 +130,49 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// The same wait by a whole, converged warp, with one verdict for all its lanes.  A role whose work is a single thread's (TMA loads,
+// MMAs) still runs its loop and its waits with the whole warp and enters elect_one() only for the instructions themselves: a lane that
+// waits on memory while the other 31 stand at the end of its branch pays about 100 clocks for it (measured with nothing else on
+// the SM: a passed wait 200 clocks for one lane and 55 to 90 for the warp, a shared load 129 and 40).  The loop is one small body
+// on purpose: an issuer's code runs once per step between the working warps' code, and every jump over a slow path costs
+// it an instruction fetch of about 100 clocks.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns = kWaitLimitNs)
+{
+    uint64_t t0 = 0;
+#pragma unroll 1
+    for (uint32_t i = 0;; ++i) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+            return true;
+        }
+        if (i >= 64u) {
+            __nanosleep(kPollSleepNs);
+            if ((i & 255u) == 255u) {
+                const uint64_t now = global_timer_ns();
+                t0 = t0 == 0 ? now : t0;
+                if (__any_sync(0xffffffffu, *abort_flag != 0 || now - t0 > limit_ns)) {
+                    return false;
+                }
+            }
+        }
+    }
+}
+
+// A whole-warp wait that is expected to be long: it looks rarely, and so costs the working warps nothing.
+__device__ __forceinline__ bool mbar_wait_lazy(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns = kWaitLimitNs)
+{
+    uint64_t t0 = 0;
+#pragma unroll 1
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        __nanosleep(200);
+        const uint64_t now = global_timer_ns();
+        t0 = t0 == 0 ? now : t0;
+        if (__any_sync(0xffffffffu, *abort_flag != 0 || now - t0 > limit_ns)) {
+            return false;
+        }
+    }
+    return true;
+}
+
 // ------------------------------------------------------------------------------- TMA
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m)
 {

@@ -71,6 +71,44 @@ def test_attention_wide_scores_and_rescale(ops):
     _check(out.cpu(), want, torch.bfloat16)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch,seq,heads", [(1, 1, 3), (1, 127, 2), (5, 129, 60), (2, 257, 80), (1, 385, 75)])
+def test_attention_edges_of_tiles_and_several_blocks_per_cta(ops, dtype, batch, seq, heads):
+    """Lengths one off a tile of 128 keys and a block of 256 queries, and more blocks than SMs, so that CTAs walk into a second and a
+    third block: its first scores are computed while the last block's sums and accumulator are still being read."""
+    g = torch.Generator().manual_seed(seq + heads)
+    qkv = _qkv(batch, seq, heads, 128, dtype, g)
+    want = _oracle(qkv, batch, seq, heads, 128)
+    out = torch.full((batch * seq, heads * 128), float("nan"), dtype=dtype, device="cuda")
+    ops.flash_attention(cu(qkv), batch, seq, heads, 128, out=out)
+    check_status()
+    _check(out.cpu(), want, dtype)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("key", [0, 15, 77, 200, 299])
+def test_attention_with_a_score_that_is_no_number(ops, bad, key):
+    """A NaN or infinite score makes its rows NaN, whichever unit computes that key's exponential and in whichever step it comes;
+    a score of -inf takes no weight unless nothing else is there; other heads are untouched."""
+    g = torch.Generator().manual_seed(11)
+    seq, heads = 300, 2
+    x = _qkv(1, seq, heads, 128, torch.bfloat16, g).reshape(seq, 3, heads, 128)
+    x[:, 0, 0, 0] = x[:, 0, 0, 0].abs() + 0.5      # head 0: every query is positive along dimension 0 ...
+    x[5, 0, 0, 0] = -x[5, 0, 0, 0]                 # ... but one
+    x[key, 1, 0, 0] = bad
+    out = torch.zeros(seq, heads * 128, dtype=torch.bfloat16, device="cuda")
+    ops.flash_attention(cu(x.reshape(seq, -1)), 1, seq, heads, 128, out=out)
+    check_status()
+    got = out.cpu().float().reshape(seq, heads, 128)
+    scores = x[:, 0, 0].double() @ x[:, 1, 0].double().t()
+    scores[:, key] = bad if bad != bad else bad * torch.sign(x[:, 0, 0, 0].double())
+    dead = (scores.max(dim=1).values == float("inf")) | torch.isnan(scores).any(dim=1)
+    assert bool(torch.isnan(got[dead, 0]).all())
+    want = torch.softmax(scores[~dead] / 128 ** 0.5, dim=-1) @ x[:, 2, 0].double()
+    _check(got[~dead, 0], want, torch.bfloat16) if bool((~dead).any()) else None
+    _check(got[:, 1], _oracle(x[:, :, 1:2].reshape(seq, -1), 1, seq, 1, 128), torch.bfloat16)
+
+
 def test_attention_e4m3_output_into_a_column_window_and_split(ops):
     """The fused quantize equals quantizing the 16-bit result (same rounding to T first, then 1 / scale and e4m3), the
     window leaves the other columns alone, and rows from `split` on land in the second output with its own scale."""
