@@ -166,6 +166,47 @@ def test_lora_down_next_to_the_quantize(ops, m, k, dt):
     assert_bit_equal(act2, act.cpu(), "second run")
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,k", [(1, 64), (33, 1600), (700, 3072)])
+@pytest.mark.parametrize("case", ["plain", "no smooth", "wide smooth", "far smooth", "wide x", "not finite", "ties"])
+def test_quantize_beside_the_low_rank_product_has_the_divisions_bits(ops, m, k, dt, case):
+    """The kernel that quantizes beside the low-rank product forms its quotients from reciprocals; the one that only quantizes divides.
+    Same codes and scales, for factors and values inside the range where that is exact, at its edges and outside it, for
+    zero groups, NaN and infinities, and for values whose quotients lie on half-integers."""
+    g = torch.Generator(device="cuda").manual_seed(m + k)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    u = lambda *s: torch.rand(*s, generator=g, device="cuda")
+    x, smooth, down = r(m, k), u(k) + 0.5, r(32, k).to(dt)
+    if case == "no smooth":
+        smooth = None
+    elif case == "wide smooth":
+        smooth = torch.exp2(40 * u(k) - 20) * torch.where(u(k) < 0.5, -1.0, 1.0)
+    elif case == "far smooth":
+        smooth = torch.exp2(140 * u(k) - 70)
+        smooth[::7] = 1.0
+    elif case == "wide x":
+        x = x * torch.exp2((60 if dt == torch.bfloat16 else 20) * (u(m, k) - 0.5))
+        x[:, ::64] = 0
+    elif case == "not finite":
+        x[u(m, k) < 0.002] = float("nan")
+        x[u(m, k) < 0.002] = float("inf")
+        x[:, :64] = 0
+    elif case == "ties":
+        smooth = torch.ones(k, device="cuda")
+        x = torch.round(x * 4) / 2
+        x[:, ::64] = 7.0
+    x = x.to(dt)
+    act = torch.empty(m, 32, device="cuda")
+    out = []
+    for low in (None, down):
+        q, s = torch.full((m, k // 2), 0xA5, dtype=torch.uint8, device="cuda"), torch.full((m, k // 64), -1.0, device="cuda")
+        ops.invoke_fused_quantize_and_lora_down_simple(None if low is None else act, q, s, x, low, smooth)
+        check_status()
+        out.append((q.cpu(), s.cpu().view(torch.int32)))
+    assert torch.equal(out[0][1], out[1][1])
+    assert torch.equal(out[0][0], out[1][0])
+
+
 @pytest.mark.parametrize("m,n,k", [(128, 128, 128), (130, 72, 192), (260, 520, 3072)])
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 def test_lora_up_added_after_the_groups(ops, m, n, k, dt):
