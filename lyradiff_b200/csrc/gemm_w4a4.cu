@@ -218,83 +218,81 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     const int num_slots = (num_kb + 3) / 4;  // scale slots per tile
 
     if (warp == 0) {
-        if (elect_one()) {
-            // -------------------------------------------------------------- TMA producer
-            int      stage = 0, issued = 0;
-            uint32_t phase = 0;
-            bool     ok = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                const int m_blk = tile % p.m_tiles;
-                const int n_blk = tile / p.m_tiles;
-                for (int kb = 0; kb < num_kb; ++kb) {
-                    if (!mbar_wait(empty_p(stage), phase ^ 1u, abort_flag)) {
-                        report_timeout(p.status, 0x1100u | (unsigned)stage);
-                        *abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t dst = packed0 + stage * kPackedStage;
-                    {
-                        mbar_arrive_expect_tx(full_p(stage), (uint32_t)kPackedStage);
-                        tma_load_2d(dst, &tmap_a, full_p(stage), kb * kPackedRowB, m_blk * kBM);
-                        tma_load_2d(dst + kPackedTile, &tmap_b, full_p(stage), kb * kPackedRowB, n_blk * kBN);
-                    }
-                    ++issued;
-                    if (++stage == kPStages) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
+        // -------------------------------------------------------------- TMA producer
+        int      stage = 0, issued = 0;
+        uint32_t phase = 0;
+        bool     ok = true;
+        for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+            const int m_blk = tile % p.m_tiles;
+            const int n_blk = tile / p.m_tiles;
+            for (int kb = 0; kb < num_kb; ++kb) {
+                if (!mbar_wait_warp(empty_p(stage), phase ^ 1u, abort_flag)) {
+                    report_timeout(p.status, 0x1100u | (unsigned)stage);
+                    *abort_flag = 1;
+                    ok = false;
+                    break;
+                }
+                const uint32_t dst = packed0 + stage * kPackedStage;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(full_p(stage), (uint32_t)kPackedStage);
+                    tma_load_2d(dst, &tmap_a, full_p(stage), kb * kPackedRowB, m_blk * kBM);
+                    tma_load_2d(dst + kPackedTile, &tmap_b, full_p(stage), kb * kPackedRowB, n_blk * kBN);
+                }
+                ++issued;
+                if (++stage == kPStages) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
             }
-            int      s  = stage;
-            uint32_t ph = phase;
-            for (int i = 0; i < kPStages && i < issued; ++i) {
-                if (s == 0) {
-                    s = kPStages;
-                    ph ^= 1u;
-                }
-                --s;
-                const uint64_t t0 = global_timer_ns();
-                while (!mbar_try_wait(full_p(s), ph)) {
-                    if (global_timer_ns() - t0 > kWaitLimitNs) {
-                        report_timeout(p.status, 0x1500u | (unsigned)s);
-                        break;
-                    }
+        }
+        int      s  = stage;
+        uint32_t ph = phase;
+        for (int i = 0; i < kPStages && i < issued; ++i) {
+            if (s == 0) {
+                s = kPStages;
+                ph ^= 1u;
+            }
+            --s;
+            const uint64_t t0 = global_timer_ns();
+            while (!mbar_try_wait(full_p(s), ph)) {
+                if (global_timer_ns() - t0 > kWaitLimitNs) {
+                    report_timeout(p.status, 0x1500u | (unsigned)s);
+                    break;
                 }
             }
         }
     } else if (warp == 1) {
-        if (elect_one()) {
-            // -------------------------------------------------------------- MMA issuer
-            // One hand-off per K block, not per group: both groups of a block go into the two partial buffers of a pair
-            // (pairs alternate between blocks) behind one commit, and the drain warps wait once for both.  A hand-off through
-            // an mbarrier costs each side a couple of hundred cycles, a group is 128 cycles of tensor work.
-            int       ustage = 0;
-            uint32_t  uphase = 0;
-            uint32_t  n      = 0;  // K-block steps issued
-            bool      ok     = true;
-            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                const int steps = num_kb + (p.lora_act != nullptr ? 1 : 0);  // the low-rank product is one more step
-                for (int kb = 0; ok && kb < steps; ++kb) {
-                    if (!mbar_wait(full_u(ustage), uphase, abort_flag)) {
-                        report_timeout(p.status, 0x1200u | (unsigned)ustage);
-                        *abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    const int q = (int)(n & 1u);
-                    if (!mbar_wait(part_empty(q), ((n >> 1) & 1u) ^ 1u, abort_flag)) {
-                        report_timeout(p.status, 0x1300u | (unsigned)q);
-                        *abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const bool     lora_step = (kb == num_kb);
-                    const int      groups    = lora_step ? 1 : min(2, p.G - 2 * kb);
-                    const uint32_t a_addr    = ustage0 + ustage * kUStage;
-                    const uint64_t adesc     = umma_desc_k_sw128(a_addr);
-                    const uint64_t bdesc     = umma_desc_k_sw128(a_addr + kOperandTile);
+        // -------------------------------------------------------------- MMA issuer
+        // One hand-off per K block, not per group: both groups of a block go into the two partial buffers of a pair
+        // (pairs alternate between blocks) behind one commit, and the drain warps wait once for both.  A hand-off through
+        // an mbarrier costs each side a couple of hundred cycles, a group is 128 cycles of tensor work.
+        int       ustage = 0;
+        uint32_t  uphase = 0;
+        uint32_t  n      = 0;  // K-block steps issued
+        bool      ok     = true;
+        for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+            const int steps = num_kb + (p.lora_act != nullptr ? 1 : 0);  // the low-rank product is one more step
+            for (int kb = 0; ok && kb < steps; ++kb) {
+                if (!mbar_wait_warp(full_u(ustage), uphase, abort_flag)) {
+                    report_timeout(p.status, 0x1200u | (unsigned)ustage);
+                    *abort_flag = 1;
+                    ok = false;
+                    break;
+                }
+                const int q = (int)(n & 1u);
+                if (!mbar_wait_warp(part_empty(q), ((n >> 1) & 1u) ^ 1u, abort_flag)) {
+                    report_timeout(p.status, 0x1300u | (unsigned)q);
+                    *abort_flag = 1;
+                    ok = false;
+                    break;
+                }
+                tc_fence_after_sync();
+                const bool     lora_step = (kb == num_kb);
+                const int      groups    = lora_step ? 1 : min(2, p.G - 2 * kb);
+                const uint32_t a_addr    = ustage0 + ustage * kUStage;
+                const uint64_t adesc     = umma_desc_k_sw128(a_addr);
+                const uint64_t bdesc     = umma_desc_k_sw128(a_addr + kOperandTile);
+                if (elect_one()) {
                     if (lora_step) {
                         // two K = 16 MMAs on 16-bit operands: the fp32 low-rank product
                         const uint32_t idesc = umma_idesc(1u, p.c_dtype == LYRAQ_BF16 ? 1u : 0u, kBM, kBN);
@@ -313,12 +311,12 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                         }
                     }
                     tc_commit(part_full(q));
-                    ++n;
                     tc_commit(empty_u(ustage));
-                    if (++ustage == kUStages) {
-                        ustage = 0;
-                        uphase ^= 1u;
-                    }
+                }
+                ++n;
+                if (++ustage == kUStages) {
+                    ustage = 0;
+                    uphase ^= 1u;
                 }
             }
         }
@@ -331,7 +329,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const int m_blk = tile % p.m_tiles;
             const int n_blk = tile / p.m_tiles;
             for (int sl = 0; sl < num_slots; ++sl) {
-                if (!__all_sync(0xffffffffu, mbar_wait(sc_empty(slot), sphase ^ 1u, abort_flag))) {
+                if (!mbar_wait_warp(sc_empty(slot), sphase ^ 1u, abort_flag)) {
                     if (lane == 0) {
                         report_timeout(p.status, 0x1800u | (unsigned)slot);
                     }
@@ -426,8 +424,8 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         bool      ok = true;
         for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
             for (int kb = 0; kb < num_kb; ++kb) {
-                bool w = mbar_wait(full_p(pstage), pphase, abort_flag);
-                w      = w && mbar_wait(empty_u(ustage), uphase ^ 1u, abort_flag);
+                bool w = mbar_wait_warp(full_p(pstage), pphase, abort_flag);
+                w      = w && mbar_wait_warp(empty_u(ustage), uphase ^ 1u, abort_flag);
                 if (!__all_sync(0xffffffffu, w)) {
                     if (lane == 0) {
                         report_timeout(p.status, 0x1400u | (unsigned)(pstage * 16 + ustage));
@@ -469,7 +467,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             if (ok && p.lora_act != nullptr) {
                 // low-rank operands: row tu of T(act) and of up, 64 bytes each, into the first four (swizzled) 16-byte
                 // pieces of the row's 128-byte line; the other four pieces are never read by the two K = 16 steps
-                if (!__all_sync(0xffffffffu, mbar_wait(empty_u(ustage), uphase ^ 1u, abort_flag))) {
+                if (!mbar_wait_warp(empty_u(ustage), uphase ^ 1u, abort_flag)) {
                     if (lane == 0) {
                         report_timeout(p.status, 0x1a00u | (unsigned)ustage);
                     }
@@ -539,7 +537,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             }
             for (int kb = 0; ok && kb < num_kb; ++kb) {
                 if ((kb & 3) == 0) {
-                    const bool got_s = mbar_wait(sc_full(slot), sphase, abort_flag);
+                    const bool got_s = mbar_wait_warp(sc_full(slot), sphase, abort_flag);
                     if (!__all_sync(0xffffffffu, got_s)) {
                         if (lane == 0) {
                             report_timeout(p.status, 0x1600u | (unsigned)slot);
@@ -553,7 +551,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 const float* sbs    = sas + kSlotGroups * kBM;
                 const int    groups = min(2, p.G - 2 * kb);
                 const int    q      = (int)(n & 1u);
-                const bool   got_p  = mbar_wait(part_full(q), (n >> 1) & 1u, abort_flag);
+                const bool   got_p  = mbar_wait_warp(part_full(q), (n >> 1) & 1u, abort_flag);
                 ++n;
                 if (!__all_sync(0xffffffffu, got_p)) {
                     if (lane == 0) {
@@ -613,7 +611,7 @@ gemm_w4a4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             if (ok && p.lora_act != nullptr) {
                 const int q  = (int)(n & 1u);
                 const int pb = 2 * q;
-                if (!__all_sync(0xffffffffu, mbar_wait(part_full(q), (n >> 1) & 1u, abort_flag))) {
+                if (!mbar_wait_warp(part_full(q), (n >> 1) & 1u, abort_flag)) {
                     if (lane == 0) {
                         report_timeout(p.status, 0x1b00u | (unsigned)pb);
                     }

@@ -21,14 +21,15 @@
 //                memory as [g][row] (ring of 2 slots); it also owns tensor memory
 //   warps 4-11   drain: warp w reads TMEM lanes 32 * (w % 4) .., 64 columns, of both row halves, so a thread owns two half rows;
 //                final epilogue
-// Measured with the rewrite included: [4608, 12288, 3072] 638 -> 489 us, [4608, 21504, 3072] 1069 -> 832 us, [4608, 3072, 12288]
-// 570 -> 456 us against gemm_w4a4_kernel; about 1300 clocks a group, of which the drain's arithmetic and loads are 1000.
+// Measured with the rewrite included: [4608, 12288, 3072] 433 us, [4608, 3072, 12288] 405, [1500, 9216, 3072] 121 (484, 441 and 131
+// with a drain that asked for a group's scales and barrier when it came to it, and issuers and producer waiting as single lanes); about
+// 1150 clocks a group.  The drain alone -- loads from tensor memory, column scales, arithmetic -- takes 674 of them.
 //
 // What shaped the drain (clocks per group and SM, [4608, 12288, 3072]): a broadcast 16-byte shared load takes the SM's one
 // shared-memory pipe two clocks, so with one row per thread the column scales cost 525 of them beside 384 for the operands of the
 // MMAs; two rows per thread halve that.  (The 16x256b form of the tensor-memory load, where a thread needs few column scales, reads
 // at a quarter of the speed of the 32x32b form.)  Loads from tensor memory run one piece ahead of the arithmetic, and the barrier of
-// the next group is tested in the middle of the current one: passing a barrier takes 230 clocks even when it is complete.
+// the next group is tested two pieces before it is needed (with test_wait: try_wait stops the warp, 449 us instead of 404).
 // The low-rank branch is one more K block per tile: T(act) [m, 32] and up [n, 32] are 64-byte rows that TMA pads to 128 with
 // zeros, two kind::f16 MMAs put the product into the next partial buffer and the drain adds it after the last group.
 // All waits are bounded (see sm100_ptx.cuh); a timeout sets the status word and every role exits.
@@ -154,6 +155,15 @@ constexpr int kHalfM       = kBM / 2;                   // rows of one MMA: an i
 constexpr int kDrainRegs   = 216;
 constexpr int kOtherRegs   = 72;
 
+// gelu_tanh_f32 of both values, operation by operation, on packed pairs ([4608, 12288, 3072] with GELU: 427 -> 411 us).
+__device__ __forceinline__ float2 gelu_tanh_pair(float2 v)
+{
+    const float2 cube = mul_f32x2(mul_f32x2(make_float2(0.044715f, 0.044715f), v), v);
+    const float2 a    = mul_f32x2(make_float2(0.7978845608028654f, 0.7978845608028654f), fma_f32x2(cube, v, v));
+    const float2 one  = add_f32x2(make_float2(1.0f, 1.0f), make_float2(tanh_approx(a.x), tanh_approx(a.y)));
+    return mul_f32x2(v, mul_f32x2(make_float2(0.5f, 0.5f), one));
+}
+
 // The value of one output pair through the epilogue, up to the last rounding.
 template<typename T>
 __device__ __forceinline__ float2 finish_pair(const Params& p, float2 v, float2 bias, bool has_bias, float2 res, bool has_res)
@@ -172,8 +182,7 @@ __device__ __forceinline__ float2 finish_pair(const Params& p, float2 v, float2 
         round_both();
     }
     if (p.gelu) {
-        v.x = gelu_tanh_f32(v.x);
-        v.y = gelu_tanh_f32(v.y);
+        v = gelu_tanh_pair(v);
         round_both();
     }
     if (has_res) {
@@ -315,109 +324,105 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const int  num_kb    = (p.K + kKBlock - 1) / kKBlock;
     const int  num_slots = (num_kb + 1) / 2;  // scale slots per tile
     const bool lora      = p.lora_act != nullptr;
+    auto give_up = [&](unsigned code) {
+        report_timeout(p.status, code);
+        *abort_flag = 1;
+    };
 
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
         if (warp == 0) {
-            if (elect_one()) {
-                // ---------------------------------------------------------- TMA producer
-                int      stage = 0, issued = 0;
-                uint32_t phase = 0;
-                bool     ok = true;
-                for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                    const int m0 = (tile % p.m_tiles) * kBM;
-                    const int n0 = (tile / p.m_tiles) * kBN;
-                    for (int kb = 0; kb < num_kb + (lora ? 1 : 0); ++kb) {
-                        if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag)) {
-                            report_timeout(p.status, 0x5100u | (unsigned)stage);
-                            *abort_flag = 1;
-                            ok = false;
-                            break;
-                        }
-                        const uint32_t dst = smem_base + stage * kStage;
+            // -------------------------------------------------------------- TMA producer
+            int      stage = 0, issued = 0;
+            uint32_t phase = 0;
+            bool     ok = true;
+            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+                const int m0 = (tile % p.m_tiles) * kBM;
+                const int n0 = (tile / p.m_tiles) * kBN;
+                for (int kb = 0; kb < num_kb + (lora ? 1 : 0); ++kb) {
+                    if (!mbar_wait_warp(empty_bar(stage), phase ^ 1u, abort_flag)) {
+                        give_up(0x5100u | (unsigned)stage);
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t dst = smem_base + stage * kStage;
+                    const bool     low = kb == num_kb;
+                    if (elect_one()) {
                         mbar_arrive_expect_tx(full_bar(stage), (uint32_t)kStage);
-                        const bool low = kb == num_kb;
                         tma_load_2d(dst, low ? &tmap_act : &tmap_a, full_bar(stage), low ? 0 : kb * kKBlock, m0);
                         tma_load_2d(dst + kATile, low ? &tmap_up : &tmap_b, full_bar(stage), low ? 0 : kb * kKBlock, n0);
-                        ++issued;
-                        if (++stage == kStages) {
-                            stage = 0;
-                            phase ^= 1u;
-                        }
+                    }
+                    ++issued;
+                    if (++stage == kStages) {
+                        stage = 0;
+                        phase ^= 1u;
                     }
                 }
-                // no copy may be in flight when the block leaves
-                int      s  = stage;
-                uint32_t ph = phase;
-                for (int i = 0; i < kStages && i < issued; ++i) {
-                    if (s == 0) {
-                        s = kStages;
-                        ph ^= 1u;
-                    }
-                    --s;
-                    const uint64_t t0 = global_timer_ns();
-                    while (!mbar_try_wait(full_bar(s), ph)) {
-                        if (global_timer_ns() - t0 > kWaitLimitNs) {
-                            report_timeout(p.status, 0x5500u | (unsigned)s);
-                            break;
-                        }
+            }
+            // no copy may be in flight when the block leaves
+            for (int i = 0; i < kStages && i < issued; ++i) {
+                if (stage == 0) {
+                    stage = kStages;
+                    phase ^= 1u;
+                }
+                --stage;
+                const uint64_t t0 = global_timer_ns();
+                while (!mbar_try_wait(full_bar(stage), phase)) {
+                    if (global_timer_ns() - t0 > kWaitLimitNs) {
+                        report_timeout(p.status, 0x5500u | (unsigned)stage);
+                        break;
                     }
                 }
             }
         } else if (warp != 2) {
-            if (elect_one()) {
-                // ---------------------------------------------------------- MMA issuer of the steps n with n & 1 == q
-                const uint32_t q     = (uint32_t)(warp >> 1);
-                const uint32_t d     = tmem_base + q * kBN;
-                int            stage = 0;
-                uint32_t       phase = 0;
-                uint32_t       n     = 0;  // steps (groups and low-rank products) of both issuers
-                bool           ok    = true;
-                const uint32_t idesc_low = umma_idesc(1u, p.c_dtype == LYRAQ_BF16 ? 1u : 0u, kHalfM, kBN);
-                for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-                    for (int kb = 0; ok && kb < num_kb + (lora ? 1 : 0); ++kb) {
-                        if (!mbar_wait(full_bar(stage), phase, abort_flag)) {
-                            report_timeout(p.status, 0x5200u | (unsigned)stage);
-                            *abort_flag = 1;
-                            ok = false;
-                            break;
-                        }
-                        const uint64_t a0     = umma_desc_k_sw128(smem_base + stage * kStage);
-                        const uint64_t a1     = umma_desc_k_sw128(smem_base + stage * kStage + kHalfM * kKBlock);
-                        const uint64_t b0     = umma_desc_k_sw128(smem_base + stage * kStage + kATile);
-                        const bool     low    = kb == num_kb;
-                        const int      groups = low ? 1 : min(2, p.G - 2 * kb);
-                        for (int g = 0; g < groups; ++g, ++n) {
-                            if ((n & 1u) != q) {
-                                continue;
-                            }
-                            // the half of tensor memory, once the drain has given it back
-                            if (!mbar_wait(part_empty(q), ((n >> 1) & 1u) ^ 1u, abort_flag)) {
-                                report_timeout(p.status, 0x5300u | q);
-                                *abort_flag = 1;
-                                ok = false;
-                                break;
-                            }
-                            tc_fence_after_sync();
-                            const uint64_t k = (uint64_t)(g * 4);  // a K step of 32 bytes is 2 in 16-byte units
+            // -------------------------------------------------------------- MMA issuer of the steps n with n & 1 == q
+            const uint32_t q     = (uint32_t)(warp >> 1);
+            const uint32_t d     = tmem_base + q * kBN;
+            int            stage = 0;
+            uint32_t       phase = 0;
+            uint32_t       n     = 0;  // steps (groups and low-rank products) of both issuers
+            bool           ok    = true;
+            const uint32_t idesc_low = umma_idesc(1u, p.c_dtype == LYRAQ_BF16 ? 1u : 0u, kHalfM, kBN);
+            for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
+                for (int kb = 0; kb < num_kb + (lora ? 1 : 0); ++kb) {
+                    const bool     low    = kb == num_kb;
+                    const int      groups = low ? 1 : min(2, p.G - 2 * kb);
+                    const int      g      = (int)((n ^ q) & 1u);   // this issuer's group of the block, if the block has it
+                    // a K step of 32 bytes is 2 in 16-byte units
+                    const uint64_t a0 = umma_desc_k_sw128(smem_base + stage * kStage) + (uint64_t)(g * 4);
+                    const uint64_t a1 = a0 + (uint64_t)((kHalfM * kKBlock) >> 4);
+                    const uint64_t b0 = a0 + (uint64_t)(kATile >> 4);
+                    ok = mbar_wait_warp(full_bar(stage), phase, abort_flag);
+                    if (ok && g < groups) {
+                        // the half of tensor memory, once the drain has given it back
+                        ok = mbar_wait_warp(part_empty(q), (((n + (uint32_t)g) >> 1) & 1u) ^ 1u, abort_flag);
+                    }
+                    if (!ok) {
+                        give_up(0x5200u | (unsigned)stage);
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    if (elect_one()) {
+                        if (g < groups) {
                             if (low) {
                                 mma_f16(d, a0, b0, idesc_low, 0u);
                                 mma_f16(d, a0 + 2, b0 + 2, idesc_low, 1u);
                                 mma_f16(d + 2 * kBN, a1, b0, idesc_low, 0u);
                                 mma_f16(d + 2 * kBN, a1 + 2, b0 + 2, idesc_low, 1u);
                             } else {
-                                mma_f8f6f4(d, a0 + k, b0 + k, kIdesc, 0u);
-                                mma_f8f6f4(d, a0 + k + 2, b0 + k + 2, kIdesc, 1u);
-                                mma_f8f6f4(d + 2 * kBN, a1 + k, b0 + k, kIdesc, 0u);
-                                mma_f8f6f4(d + 2 * kBN, a1 + k + 2, b0 + k + 2, kIdesc, 1u);
+                                mma_f8f6f4(d, a0, b0, kIdesc, 0u);
+                                mma_f8f6f4(d, a0 + 2, b0 + 2, kIdesc, 1u);
+                                mma_f8f6f4(d + 2 * kBN, a1, b0, kIdesc, 0u);
+                                mma_f8f6f4(d + 2 * kBN, a1 + 2, b0 + 2, kIdesc, 1u);
                             }
                             tc_commit(part_full(q));
                         }
                         tc_commit(empty_bar(stage));   // each issuer once per block, after its own MMAs on it (if any)
-                        if (++stage == kStages) {
-                            stage = 0;
-                            phase ^= 1u;
-                        }
+                    }
+                    n += (uint32_t)groups;
+                    if (++stage == kStages) {
+                        stage = 0;
+                        phase ^= 1u;
                     }
                 }
             }
@@ -432,11 +437,8 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 const int m0 = (tile % p.m_tiles) * kBM;
                 const int n0 = (tile / p.m_tiles) * kBN;
                 for (int sl = 0; sl < num_slots; ++sl) {
-                    if (!__all_sync(0xffffffffu, mbar_wait(sc_empty(slot), sphase ^ 1u, abort_flag))) {
-                        if (lane == 0) {
-                            report_timeout(p.status, 0x5800u | (unsigned)slot);
-                        }
-                        *abort_flag = 1;
+                    if (!mbar_wait_warp(sc_empty(slot), sphase ^ 1u, abort_flag)) {
+                        give_up(0x5800u | (unsigned)slot);
                         ok = false;
                         break;
                     }
@@ -511,17 +513,12 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         int            slot = 0;
         uint32_t       sphase = 0;
         uint32_t       n = 0;          // steps (groups and low-rank products) drained
-        bool           ready = false;  // the barrier of step n was seen complete ahead of time
         bool           ok = true;
-        auto wait_step = [&]() {
-            if (!__all_sync(0xffffffffu, ready || mbar_wait(part_full(n & 1u), (n >> 1) & 1u, abort_flag))) {
-                if (lane == 0) {
-                    report_timeout(p.status, 0x5700u);
-                }
-                *abort_flag = 1;
+        auto wait_step = [&](bool ready) {   // ready: the barrier was seen complete ahead of time
+            if (!__all_sync(0xffffffffu, ready) && !mbar_wait_warp(part_full(n & 1u), (n >> 1) & 1u, abort_flag)) {
+                give_up(0x5700u);
                 ok = false;
             }
-            ready = false;
             tc_fence_after_sync();
             return tmem_base + lane_addr + (n & 1u) * kBN;
         };
@@ -549,38 +546,51 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 acc[0][i] = make_float2(0.0f, 0.0f);
                 acc[1][i] = make_float2(0.0f, 0.0f);
             }
+            // What a group needs first is fetched while the last piece of the group before is rescaled, and its barriers are looked at
+            // in that group, so that a group begins without a pause: the drain warps of a scheduler run in step, and whatever one waits
+            // for, both wait for.
             uint32_t pcs[2][16];
-            uint32_t next_addr = wait_step();
+            float4   sb[2][4];
+            float2   sa[2];
+            auto slot_scales = [&](int sl, int in_slot) {
+                return reinterpret_cast<const float*>(gen_base + kScaleOffset + sl * kScaleSlot) + in_slot * kBM + quad * 32 + lane;
+            };
+            auto slot_columns = [&](int sl, int in_slot) {
+                return reinterpret_cast<const float4*>(gen_base + kScaleOffset + sl * kScaleSlot + (kSlotGroups * kBM + in_slot * kBN + part * kCols) * 4);
+            };
+            auto wait_scales = [&](int sl, uint32_t ph) {
+                if (!mbar_wait_warp(sc_full(sl), ph, abort_flag)) {
+                    give_up(0x5600u | (unsigned)sl);
+                    ok = false;
+                }
+            };
+            wait_scales(slot, sphase);
+            uint32_t t_addr = ok ? wait_step(false) : 0u;
             if (!ok) {
                 break;
             }
-            tmem_ld_32x16(next_addr, pcs[0]);
+            tmem_ld_32x16(t_addr, pcs[0]);
+            const float*  sas = slot_scales(slot, 0);
+            const float4* sb4 = slot_columns(slot, 0);
+            sa[0] = make_float2(sas[0], sas[0]);
+            sa[1] = make_float2(sas[kHalfM], sas[kHalfM]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                sb[0][j] = sb4[j];
+            }
+            int in_slot = 0;
 #pragma unroll 1
             for (int g = 0; g < p.G; ++g) {
-                const int in_slot = g % kSlotGroups;
-                if (in_slot == 0) {
-                    if (!__all_sync(0xffffffffu, mbar_wait(sc_full(slot), sphase, abort_flag))) {
-                        if (lane == 0) {
-                            report_timeout(p.status, 0x5600u | (unsigned)slot);
-                        }
-                        *abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                }
-                const float*  sas = reinterpret_cast<const float*>(gen_base + kScaleOffset + slot * kScaleSlot);
-                const float4* sb4 = reinterpret_cast<const float4*>(sas + kSlotGroups * kBM + in_slot * kBN + part * kCols);
-                sas += in_slot * kBM + quad * 32 + lane;
-                const float2 sa[2] = {make_float2(sas[0], sas[0]), make_float2(sas[kHalfM], sas[kHalfM])};
-                const uint32_t t_addr = next_addr;
+                const bool    more  = g + 1 < p.G;
+                const bool    leave = in_slot == kSlotGroups - 1 || !more;   // the slot's last group
+                const int     slot2 = !leave ? slot : (slot + 1 == kSSlots ? 0 : slot + 1);
+                float2        sa2[2];
+                bool          ready     = false;
+                const float4* nb4       = sb4;
+                uint32_t      next_addr = t_addr;
                 // piece i: 16 columns 16 (i / 2) .. of row half i & 1; the load of piece i + 1 (of the next group's first one, at
                 // the end) is in flight while piece i is rescaled, and the column scales of the next 16 columns are fetched a piece
                 // ahead as well
-                float4 sb[2][4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    sb[0][j] = sb4[j];
-                }
 #pragma unroll
                 for (int i = 0; i < kCols / 8; ++i) {
                     const int h = i & 1, c = i >> 1;
@@ -589,20 +599,35 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                         tmem_ld_32x16(t_addr + (uint32_t)(((i + 1) & 1) * 2 * kBN + ((i + 1) >> 1) * 16), pcs[(i + 1) & 1]);
                     } else {
                         release_step();   // all of the group is in registers
-                        if (g + 1 < p.G) {
-                            next_addr = wait_step();
+                        if (more) {
+                            next_addr = wait_step(ready);
                             if (ok) {
                                 tmem_ld_32x16(next_addr, pcs[0]);
                             }
                         }
                     }
-                    if (i == kCols / 16) {
-                        ready = mbar_test_wait(part_full((n + 1) & 1u), ((n + 1) >> 1) & 1u);
+                    if (i == kCols / 8 - 2) {
+                        ready = mbar_test_wait(part_full((n + 1) & 1u), ((n + 1) >> 1) & 1u);   // test_wait: try_wait would stop here
                     }
-                    if (h == 1 && c + 1 < kCols / 16) {
+                    if (i == kCols / 16 && leave && more) {
+                        wait_scales(slot2, slot2 == 0 ? sphase ^ 1u : sphase);
+                    }
+                    if (h == 1) {
+                        if (c + 1 < kCols / 16) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            sb[(c + 1) & 1][j] = sb4[(c + 1) * 4 + j];
+                            for (int j = 0; j < 4; ++j) {
+                                sb[(c + 1) & 1][j] = sb4[(c + 1) * 4 + j];
+                            }
+                        } else {
+                            const int    in2 = leave ? 0 : in_slot + 1;
+                            const float* na  = slot_scales(slot2, in2);
+                            nb4              = slot_columns(slot2, in2);
+                            sa2[0]           = make_float2(na[0], na[0]);
+                            sa2[1]           = make_float2(na[kHalfM], na[kHalfM]);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                sb[0][j] = nb4[j];
+                            }
                         }
                     }
                     const uint32_t* pc = pcs[i & 1];
@@ -621,19 +646,22 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 if (!ok) {
                     break;
                 }
-                if (in_slot == kSlotGroups - 1 || g == p.G - 1) {
+                if (leave) {
                     __syncwarp();
                     if (lane == 0) {
                         mbar_arrive(sc_empty(slot));
                     }
-                    if (++slot == kSSlots) {
-                        slot = 0;
-                        sphase ^= 1u;
-                    }
+                    slot = slot2;
+                    sphase ^= slot2 == 0 ? 1u : 0u;
                 }
+                in_slot = leave ? 0 : in_slot + 1;
+                sb4     = nb4;
+                t_addr  = next_addr;
+                sa[0]   = sa2[0];
+                sa[1]   = sa2[1];
             }
             if (ok && lora) {
-                const uint32_t t_addr = wait_step();
+                const uint32_t t_addr = wait_step(false);
                 if (ok) {
 #pragma unroll
                     for (int i = 0; i < kCols / 8; ++i) {
