@@ -15,6 +15,7 @@ struct Params {
     const void*   sb;
     int           sb_is_f16;
     int           scale_vec_ok;  // G % 4 == 0 and 16-byte aligned scale arrays: 16-byte scale loads are legal
+    int           scale_tma;     // wide kernel: both scale arrays can be addressed by TMA
     void*         D;
     int           c_dtype;
     const void*   bias;

@@ -17,13 +17,14 @@
 //   warp 0       TMA producer: A (256 x 128 B) and B (128 x 128 B) tiles of one K block = 2 groups, ring of 3 stages
 //   warps 1, 3   MMA issuers of the even and the odd steps: a group's two products [128 x 128] (rows 0-127 and 128-255) into the
 //                step's half of tensor memory, one commit per group; one thread that issued all of them took 900 clocks a group
-//   warp 2       scale loader: every two K blocks (4 groups) it transposes sa[m, g] and sb[n, g] of the tile into shared
-//                memory as [g][row] (ring of 2 slots); it also owns tensor memory
+//   warp 2       scale loader: every two K blocks (4 groups) it puts sa[m, g] and sb[n, g] of the tile into shared memory as
+//                [g][row] (ring of 2 slots), by way of TMA where the arrays allow that; it also owns tensor memory
 //   warps 4-11   drain: warp w reads TMEM lanes 32 * (w % 4) .., 64 columns, of both row halves, so a thread owns two half rows;
 //                final epilogue
-// Measured with the rewrite included: [4608, 12288, 3072] 433 us, [4608, 3072, 12288] 405, [1500, 9216, 3072] 121 (484, 441 and 131
-// with a drain that asked for a group's scales and barrier when it came to it, and issuers and producer waiting as single lanes); about
-// 1150 clocks a group.  The drain alone -- loads from tensor memory, column scales, arithmetic -- takes 674 of them.
+// Measured with the rewrite included: [4608, 12288, 3072] 416 us, [4608, 3072, 12288] 381, [1500, 9216, 3072] 115; 430, 406 and 120
+// with scales loaded by the lanes (16 bytes of 32 rows per instruction, a shared-memory-pipe pass each); 484, 441 and 131 with, besides, a
+// drain that asked for a group's scales and barrier when it came to it, and issuers and producer waiting as single lanes.  About 1060
+// clocks a group; the drain alone -- loads from tensor memory, column scales, arithmetic -- takes 674 of them.
 //
 // What shaped the drain (clocks per group and SM, [4608, 12288, 3072]): a broadcast 16-byte shared load takes the SM's one
 // shared-memory pipe two clocks, so with one row per thread the column scales cost 525 of them beside 384 for the operands of the
@@ -144,7 +145,9 @@ constexpr int kScaleSlot   = kSlotGroups * (kBM + kBN) * 4;   // sas[4][256] the
 constexpr int kBox         = 32 * 128;                  // a TMA store box: 32 rows x 128 bytes, 128-byte swizzle
 constexpr int kBoxBytes    = 2 * kBox;                  // per drain warp: one per row half
 constexpr int kScaleOffset = kStages * kStage;
-constexpr int kOutOffset   = kScaleOffset + kSSlots * kScaleSlot;
+constexpr int kRawBlock    = 128 * 16;                  // 128 rows x 4 group scales as TMA brings them, two buffers
+constexpr int kRawOffset   = kScaleOffset + kSSlots * kScaleSlot;
+constexpr int kOutOffset   = kRawOffset + 2 * kRawBlock;
 constexpr int kBiasOffset  = kOutOffset + kDrainWarps * kBoxBytes;   // 128 bytes per drain warp: the bias of its columns
 constexpr int kBarOffset   = kBiasOffset + kDrainWarps * 128;
 constexpr int kSmemTotal   = kBarOffset + 256 + 1024;
@@ -266,10 +269,23 @@ __device__ __forceinline__ void store_block_any(const Params& p, const float2* a
     }
 }
 
+// Waits, bounded, for a copy that was asked for.
+__device__ __forceinline__ void settle(uint32_t bar, uint32_t parity, unsigned int* status, unsigned code)
+{
+    const uint64_t t0 = global_timer_ns();
+    while (!mbar_try_wait(bar, parity)) {
+        if (global_timer_ns() - t0 > kWaitLimitNs) {
+            report_timeout(status, code);
+            break;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const __grid_constant__ CUtensorMap tmap_act, const __grid_constant__ CUtensorMap tmap_up,
-                      const __grid_constant__ CUtensorMap tmap_d, const Params p)
+                      const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_sa,
+                      const __grid_constant__ CUtensorMap tmap_sb, const Params p)
 {
     constexpr uint32_t kTmemCols = 4 * kBN;
     constexpr uint32_t kIdesc    = umma_idesc(1u, 0u, kHalfM, kBN);
@@ -284,7 +300,8 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     auto part_empty = [&](uint32_t b) { return bars + 8u * (2 * kStages + 2 + b); };
     auto sc_full    = [&](int s) { return bars + 8u * (2 * kStages + 4 + s); };
     auto sc_empty   = [&](int s) { return bars + 8u * (2 * kStages + 4 + kSSlots + s); };
-    constexpr int kNumBars   = 2 * kStages + 4 + 2 * kSSlots;
+    auto raw_full   = [&](int b) { return bars + 8u * (2 * kStages + 4 + 2 * kSSlots + b); };
+    constexpr int kNumBars   = 2 * kStages + 6 + 2 * kSSlots;
     uint32_t*     tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + kBarOffset + 8 * kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -305,6 +322,8 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             mbar_init(sc_full(s), 1);
             mbar_init(sc_empty(s), kDrainWarps);
         }
+        mbar_init(raw_full(0), 1);
+        mbar_init(raw_full(1), 1);
         *abort_flag = 0;
         fence_barrier_init();
         prefetch_tensormap(&tmap_a);
@@ -366,13 +385,7 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                     phase ^= 1u;
                 }
                 --stage;
-                const uint64_t t0 = global_timer_ns();
-                while (!mbar_try_wait(full_bar(stage), phase)) {
-                    if (global_timer_ns() - t0 > kWaitLimitNs) {
-                        report_timeout(p.status, 0x5500u | (unsigned)stage);
-                        break;
-                    }
-                }
+                settle(full_bar(stage), phase, p.status, 0x5500u | (unsigned)stage);
             }
         } else if (warp != 2) {
             // -------------------------------------------------------------- MMA issuer of the steps n with n & 1 == q
@@ -426,8 +439,92 @@ gemm_w4a4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                     }
                 }
             }
+        } else if (p.scale_tma) {
+            // -------------------------------------------------------------- scale loader (warp 2), scales that TMA can address
+            // A slot is three blocks of 128 rows x 4 groups (rows 0-127 and 128-255 of A, the columns of B), which TMA fetches two blocks
+            // ahead as they lie in memory, 16 bytes a row; a lane turns its four rows' pieces into [g][row].
+            const int tiles_here = (num_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+            const int blocks     = tiles_here * num_slots * 3;
+            int       i_tile = blockIdx.x, i_slot = 0, i_part = 0;   // the block to ask for next
+            auto ask = [&](int j) {
+                if (j < blocks && elect_one()) {
+                    const int      m0  = (i_tile % p.m_tiles) * kBM, n0 = (i_tile / p.m_tiles) * kBN;
+                    const uint32_t dst = smem_base + kRawOffset + (j & 1) * kRawBlock;
+                    mbar_arrive_expect_tx(raw_full(j & 1), (uint32_t)kRawBlock);
+                    if (i_part < 2) {
+                        tma_load_2d(dst, &tmap_sa, raw_full(j & 1), i_slot * kSlotGroups * 4, m0 + i_part * 128);
+                    } else {
+                        // 16-bit scales: the 16 bytes hold this slot's four groups and a neighbour's
+                        tma_load_2d(dst, &tmap_sb, raw_full(j & 1), p.sb_is_f16 ? (i_slot & ~1) * kSlotGroups * 2 : i_slot * kSlotGroups * 4, n0);
+                    }
+                }
+                if (++i_part == 3) {
+                    i_part = 0;
+                    if (++i_slot == num_slots) {
+                        i_slot = 0;
+                        i_tile += (int)gridDim.x;
+                    }
+                }
+            };
+            ask(0);
+            ask(1);
+            int      slot = 0, part = 0, s_tile = 0, asked = min(blocks, 2);
+            uint32_t sphase = 0;
+            for (int j = 0; j < blocks; ++j) {
+                if ((part == 0 && !mbar_wait_warp(sc_empty(slot), sphase ^ 1u, abort_flag)) ||
+                    !mbar_wait_warp(raw_full(j & 1), (uint32_t)((j >> 1) & 1), abort_flag)) {
+                    give_up(0x5800u | (unsigned)slot);
+                    break;
+                }
+                const uint8_t* raw  = gen_base + kRawOffset + (j & 1) * kRawBlock;
+                float*         dst  = reinterpret_cast<float*>(gen_base + kScaleOffset + slot * kScaleSlot) + (part < 2 ? part * 128 : kSlotGroups * kBM) + lane;
+                const int      step = part < 2 ? kBM : kBN;
+                const bool     half = part == 2 && p.sb_is_f16;
+                Vec16          v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    v[i] = *reinterpret_cast<const Vec16*>(raw + (i * 32 + lane) * 16);
+                }
+                __syncwarp();
+                asked += j + 2 < blocks ? 1 : 0;
+                ask(j + 2);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float x[4];
+                    if (half) {
+                        const float2 lo = Pair<__half>::to_f32((s_tile & 1) ? v[i].w[2] : v[i].w[0]);
+                        const float2 hi = Pair<__half>::to_f32((s_tile & 1) ? v[i].w[3] : v[i].w[1]);
+                        x[0] = lo.x; x[1] = lo.y; x[2] = hi.x; x[3] = hi.y;
+                    } else {
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) {
+                            x[g] = __uint_as_float(v[i].w[g]);
+                        }
+                    }
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        dst[g * step + i * 32] = x[g];
+                    }
+                }
+                if (++part == 3) {
+                    part = 0;
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(sc_full(slot));
+                    }
+                    if (++slot == kSSlots) {
+                        slot = 0;
+                        sphase ^= 1u;
+                    }
+                    s_tile = s_tile + 1 == num_slots ? 0 : s_tile + 1;   // slot number inside its tile
+                }
+            }
+            // no copy may be in flight when the block leaves: block j is the (j >> 1)-th of its buffer
+            for (int j = max(0, asked - 2); j < asked; ++j) {
+                settle(raw_full(j & 1), (uint32_t)((j >> 1) & 1), p.status, 0x5900u | (unsigned)(j & 1));
+            }
         } else {
-            // -------------------------------------------------------------- scale loader (warp 2)
+            // -------------------------------------------------------------- scale loader (warp 2), any scales
             constexpr int kRowSets = (kBM + kBN) / 32;   // sets of 32 rows
             constexpr int kBatch   = 6;                  // sets whose loads are in flight together
             int      slot = 0;
@@ -790,6 +887,20 @@ int launch_wide(Params p, const uint8_t* A, const uint8_t* B, void* workspace, i
             return st;
         }
     }
+    CUtensorMap tsa = ta, tsb = ta;   // never read where the lanes load the scales
+    // TMA wants 16-byte rows: pitches that are multiples of 16 bytes, from aligned arrays
+    p.scale_tma = (p.G & (p.sb_is_f16 ? 7 : 3)) == 0 && aligned16(p.sa) && aligned16(p.sb) ? 1 : 0;
+    if (p.scale_tma) {
+        const uint64_t sa_row = (uint64_t)p.G * 4, sb_row = (uint64_t)p.G * (p.sb_is_f16 ? 2 : 4);
+        st = make_tmap_bytes_2d(&tsa, p.sa, m, sa_row, sa_row, 128, 16, false);
+        if (st != LYRAQ_OK) {
+            return st;
+        }
+        st = make_tmap_bytes_2d(&tsb, p.sb, n, sb_row, sb_row, 128, 16, false);
+        if (st != LYRAQ_OK) {
+            return st;
+        }
+    }
     const long  tiles = (long)p.m_tiles * p.n_tiles;
     const int   grid  = (int)(tiles < sms ? tiles : sms);
     static bool smem_raised[64] = {};
@@ -799,7 +910,7 @@ int launch_wide(Params p, const uint8_t* A, const uint8_t* B, void* workspace, i
         return st;
     }
     return cuda_status(launch_kernel(wide::gemm_w4a4_wide_kernel, (unsigned)grid, (unsigned)wide::kThreads, (size_t)wide::kSmemTotal,
-                                     stream, 1u, ta, tb, tact, tup, td, p),
+                                     stream, 1u, ta, tb, tact, tup, td, tsa, tsb, p),
                        "cudaLaunchKernelEx(gemm_w4a4_wide_kernel)");
 }
 
