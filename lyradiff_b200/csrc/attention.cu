@@ -100,12 +100,13 @@ __device__ __forceinline__ float ex2_approx(float x)
 
 // 2^x of two values on the FMA and ALU pipes: x = n + f with n an integer and f in [-1/2, 1/2]; 2^f from its minimax polynomial of
 // degree 5 (Remez exchange on the relative error: 7.5e-8 in exact arithmetic, 2.1e-7 evaluated in fp32, which is what ex2.approx
-// has), and n added to the exponent.  x below -126 gives 2^-126.  NaN and infinity do not come through: the caller looks for them
-// in the row's maximum.
+// has), and n added to the exponent.  x of -127 and below gives the smallest subnormal, which both 16-bit types round to a weight of zero,
+// as ex2.approx.ftz does: such a key adds nothing to O, whatever its value row holds.  (Between -126 and -127 the result is some subnormal.)
+// NaN and infinity do not come through: the caller looks for them in the row's maximum.
 __device__ __forceinline__ float2 ex2_poly(float2 x)
 {
     const float  magic = 12582912.0f;   // 1.5 * 2^23: the sum's low mantissa bits are n
-    x                  = make_float2(fmaxf(x.x, -126.0f), fmaxf(x.y, -126.0f));
+    x                  = make_float2(fmaxf(x.x, -127.0f), fmaxf(x.y, -127.0f));
     const float2 t     = add_f32x2(x, make_float2(magic, magic));
     const float2 n     = add_f32x2(t, make_float2(-magic, -magic));
     const float2 f     = fma_f32x2(n, make_float2(-1.0f, -1.0f), x);

@@ -109,6 +109,29 @@ def test_attention_with_a_score_that_is_no_number(ops, bad, key):
     _check(got[:, 1], _oracle(x[:, :, 1:2].reshape(seq, -1), 1, seq, 1, 128), torch.bfloat16)
 
 
+@pytest.mark.parametrize("value", [1e38, float("inf")])
+@pytest.mark.parametrize("key", [13, 14, 15, 31, 126, 286])
+def test_attention_key_whose_weight_underflows(ops, key, value):
+    """A key far below the maximum has a weight of zero, whichever unit computes its exponential: its value row adds nothing
+    however large it is (1e38 would still show through a weight of 2^-126), and an infinite one gives zero times infinity."""
+    g = torch.Generator().manual_seed(key)
+    seq = 300
+    x = _qkv(1, seq, 1, 128, torch.bfloat16, g).reshape(seq, 3, 1, 128)
+    x[:, 0, 0, 0] = 40.0
+    x[:, 1, 0, 0] = 0.0
+    x[key, 1, 0, 0] = -400.0                       # score -16000 / sqrt(128), about 2000 units of log2 below the others
+    x[key, 2, 0, 5] = value
+    out = torch.zeros(seq, 128, dtype=torch.bfloat16, device="cuda")
+    ops.flash_attention(cu(x.reshape(seq, -1)), 1, seq, 1, 128, out=out)
+    check_status()
+    got, want = out.cpu(), _oracle(x.reshape(seq, -1), 1, seq, 1, 128)
+    assert bool(torch.isnan(got[:, 5]).all()) == (value == float("inf"))
+    if value == float("inf"):
+        assert bool(torch.isnan(want[:, 5]).all())
+        got, want = torch.cat([got[:, :5], got[:, 6:]], 1), torch.cat([want[:, :5], want[:, 6:]], 1)
+    _check(got, want, torch.bfloat16)
+
+
 def test_attention_e4m3_output_into_a_column_window_and_split(ops):
     """The fused quantize equals quantizing the 16-bit result (same rounding to T first, then 1 / scale and e4m3), the
     window leaves the other columns alone, and rows from `split` on land in the second output with its own scale."""
