@@ -345,7 +345,8 @@ LYRAQ_API int lyraq_gemm_fp8_qk_rope(const uint8_t* X, const float* s_x, const u
  * Replaces FlashAttention2Layer<T>::forward (src/lyradiff/layers/flash_attn2/flash_attn2.cu:59-118, called at
  * layers/flux_single_attention_processor/FluxSingleAttentionFP8Processor.cc:213 and
  * layers/flux_attention_processor/FluxAttentionFP8Processor.cc:274) and the e4m3 cast of its output
- * (FluxSingleTransformerFP8Block.cc:254, FluxAttnPostFP8Processor.cc:135,168). */
+ * (FluxSingleTransformerFP8Block.cc:254, FluxAttnPostFP8Processor.cc:135,168).  softmax_scale may be any number: zero gives the mean of
+ * the values. */
 LYRAQ_API int lyraq_attention(void* out, int out_dtype, size_t out_ld, const float* out_scale, void* out2, size_t out2_ld,
                               const float* out2_scale, size_t split, const void* qkv, int dtype, size_t batch, size_t seq_len,
                               int heads, int head_dim, float softmax_scale, void* stream);

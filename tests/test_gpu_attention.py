@@ -109,6 +109,21 @@ def test_attention_with_a_score_that_is_no_number(ops, bad, key):
     _check(got[:, 1], _oracle(x[:, :, 1:2].reshape(seq, -1), 1, seq, 1, 128), torch.bfloat16)
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.05, -0.7, 0.3])
+@pytest.mark.parametrize("seq,spread", [(1, 1.0), (64, 1.0), (127, 1.0), (128, 1.0), (192, 1.0), (300, 6.0)])
+def test_attention_with_any_softmax_scale(ops, scale, seq, spread):
+    """A scale of zero is a plain mean of the values, a negative one prefers the lowest scores; keys past the end of the sequence take
+    no weight under either.  (The scaled scores of spread 6 and scale -0.7 reach far past the exponent range.)"""
+    g = torch.Generator().manual_seed(seq)
+    qkv = _qkv(1, seq, 2, 128, torch.bfloat16, g, spread=spread)
+    x = qkv.double().reshape(seq, 3, 2, 128).permute(1, 2, 0, 3)
+    want = torch.softmax(x[0] @ x[1].transpose(1, 2) * scale, dim=-1) @ x[2]
+    out = torch.full((seq, 256), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.flash_attention(cu(qkv), 1, seq, 2, 128, out=out, softmax_scale=scale)
+    check_status()
+    _check(out.cpu(), want.permute(1, 0, 2).reshape(seq, 256), torch.bfloat16)
+
+
 @pytest.mark.parametrize("value", [1e38, float("inf")])
 @pytest.mark.parametrize("key", [13, 14, 15, 31, 126, 286])
 def test_attention_key_whose_weight_underflows(ops, key, value):
