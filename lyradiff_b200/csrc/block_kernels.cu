@@ -4,6 +4,8 @@
 //     proj_out, so that attention output and MLP activation are never concatenated in 16-bit form),
 //   - gate * y + residual (the block's output).
 // All are HBM-bound streaming kernels with 16-byte accesses; arithmetic follows the reference's rounding steps.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace lyraq {
@@ -15,12 +17,15 @@ int device_sm_count();  // gemm_dense.cu
 // (src/lyradiff/kernels/rope/flux_apply_rope.cu:8-76): inv = rsqrt(mean(x^2) + eps) in fp32; t = T(x * inv);
 // t = T(t * scale); out.x = T(T(t.x * r0.x) + T(t.y * r0.y)); out.y = T(T(t.x * r1.x) + T(t.y * r1.y)); V heads are copied.
 //
-// A block takes a token at a time, so the rotation of a lane's four pairs and the norm weights stay in registers over the heads and no
-// index is divided; three vectors per thread are in flight (the q and k heads of 24 x 128 are exactly that).  Bound by memory: 113 MB
-// at 4608 tokens x 24 heads in place, where it takes 16.9 us (30.8 with a flat index over all vectors, two 64-bit divisions each).
-template<typename T, int LANES>
-__global__ void __launch_bounds__(256) rmsnorm_rope_kernel(T* out, const T* qkv, const T* scale, const T* rope, float eps,
-                                                           size_t tokens, int seq_len, int heads)
+// A token's heads are taken by threads that each keep the same four pairs, so the rotation and the norm weights stay in registers over the
+// heads and no index is divided; three vectors per thread are in flight.  Bound by memory: 113 MB at 4608 tokens x 24 heads in
+// place, where it takes 16.9 us (30.8 with a flat index over all vectors, two 64-bit divisions each).  rope_split chooses the threads of a token.
+//
+// THREADS > 0: a block of THREADS takes a token at a time.  THREADS = 0: a block of 256 has 2^tpt_log2 threads to a token, several tokens at
+// a time where that leaves room, and `chunks` blocks share a token.
+template<typename T, int LANES, int THREADS>
+__global__ void __launch_bounds__(THREADS > 0 ? THREADS : 256) rmsnorm_rope_kernel(T* out, const T* qkv, const T* scale, const T* rope,
+                                                                                   float eps, size_t tokens, int heads, int tpt_log2, int chunks)
 {
     using P2 = Pair<T>;
     grid_launch_dependents();
@@ -33,7 +38,18 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(T* out, const T* qkv,
     const size_t  pitch    = (size_t)3 * heads * kHeadDim;
     const Vec16   sc_q     = ld_nc_16_keep(scale + part * 8);
     const Vec16   sc_k     = ld_nc_16_keep(scale + kHeadDim + part * 8);
-    for (size_t tok = blockIdx.x; tok < tokens; tok += gridDim.x) {
+    constexpr bool kSplit  = THREADS == 0;
+    const int     tpt      = kSplit ? 1 << tpt_log2 : THREADS;
+    const int     mine     = kSplit ? (int)threadIdx.x & (tpt - 1) : (int)threadIdx.x;
+    const unsigned blk     = kSplit ? blockIdx.x / (unsigned)chunks : blockIdx.x, blks = kSplit ? gridDim.x / (unsigned)chunks : gridDim.x;
+    const int     first    = (kSplit ? (int)(blockIdx.x - blk * (unsigned)chunks) * tpt : 0) + mine;    // of the token's vectors
+    const int     step     = kSplit ? tpt * chunks : THREADS;
+    const size_t  sub      = kSplit ? threadIdx.x >> tpt_log2 : 0;
+    const size_t  at_once  = kSplit ? 256u >> tpt_log2 : 1;
+    for (size_t t0 = blk * at_once; t0 < tokens; t0 += blks * at_once) {
+        const bool   live = !kSplit || t0 + sub < tokens;
+        const size_t tok  = live ? t0 + sub : t0;
+        const int    n    = live ? n_vec : 0;
         // rope: [tokens, head_dim / 2, 2, 2]; this thread's 4 pairs are 16 consecutive values
         const T*    rp  = rope + tok * (size_t)(kHeadDim * 2) + part * 16;
         const Vec16 r0  = ld_nc_16_keep(rp);
@@ -41,19 +57,23 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(T* out, const T* qkv,
         const T*    src = qkv + tok * pitch;
         T*          dst = out + tok * pitch;
         // every lane of a warp takes part in the shuffles: those past the end reduce zeros and store nothing
-        for (int v0 = (int)threadIdx.x; v0 - (int)threadIdx.x < n_vec; v0 += kFlight * 256) {
+        for (int v0 = first; v0 - mine < n_vec; v0 += kFlight * step) {
             uint4 raw[kFlight];
 #pragma unroll
             for (int u = 0; u < kFlight; ++u) {
+                const int vi = v0 + u * step;
                 raw[u] = make_uint4(0u, 0u, 0u, 0u);
-                if (v0 + u * 256 < n_vec) {
+                if (vi < n) {
                     // an ordered plain load, not the read-only (.nc) path: with out == qkv this kernel writes what it reads
-                    raw[u] = ld_u32x4(reinterpret_cast<const uint4*>(src + (size_t)(v0 + u * 256) * 8));
+                    raw[u] = ld_u32x4(reinterpret_cast<const uint4*>(src + (size_t)vi * 8));
                 }
             }
 #pragma unroll
             for (int u = 0; u < kFlight; ++u) {
-                const int vi = v0 + u * 256;
+                if (kSplit && u > 0 && v0 - mine + u * step >= n_vec) {
+                    break;
+                }
+                const int vi = v0 + u * step;
                 Vec16     x;
                 x.w[0] = raw[u].x; x.w[1] = raw[u].y; x.w[2] = raw[u].z; x.w[3] = raw[u].w;
                 float f[8];
@@ -81,12 +101,46 @@ __global__ void __launch_bounds__(256) rmsnorm_rope_kernel(T* out, const T* qkv,
                         x.w[j]          = P2::from_f32(pa.x + pa.y, pb.x + pb.y);  // fp32 sum of two T values, rounded once = T add
                     }
                 }
-                if (vi < n_vec) {
+                if (vi < n) {
                     st_16(dst + (size_t)vi * 8, x);
                 }
             }
         }
     }
+}
+
+// Threads of a token.  The q and k heads of 24 x 128 are three vectors for each of 256 threads, with the v heads (out of place) 384, and more
+// heads go through such a block in turns.  With fewer such a block idles, so several tokens share it, still with three vectors a thread:
+// up to 192 vectors always, up to 384 where there are more tokens than blocks.  And where all vectors fit the chip at a few hundred
+// per SM a call is latency: a vector per thread.  Measured against 256 threads to every token and against the flat index: 65536 tokens x
+// 1 head x 64 in place 114 / 12.0 us, here 7.3; 4608 x 2 x 128 10.0 / 4.4, 3.0; 4608 x 12 x 128 12.5 / 15.4, 10.1; out of place 1 x 24 x 128
+// 2.3 / 1.7, 1.75, 77 x 24 x 128 2.7 / 2.7, 2.15, 256 x 24 x 128 3.9 / 3.4, 3.0.
+struct RopeSplit {
+    int      threads;            // of the kernel's template: 0, 256 or 384
+    int      tpt_log2, chunks;
+    unsigned grid;
+};
+static RopeSplit rope_split(size_t tokens, int heads, int lanes, bool in_place, int sms)
+{
+    const size_t n_vec = (size_t)heads * (size_t)lanes * (in_place ? 2 : 3);
+    const bool   few   = n_vec <= 192 || (n_vec <= 384 && tokens > (size_t)sms * 8);
+    const bool   brief = few ? n_vec <= 256 && tokens * n_vec <= (size_t)sms * 1024 : n_vec > 768 && tokens * n_vec <= (size_t)sms * 256;
+    RopeSplit    r{0, 3, 1, 0u};
+    size_t       blocks = tokens;
+    if (few || brief) {
+        const size_t want = brief ? n_vec : (n_vec + 2) / 3;
+        while (r.tpt_log2 < 8 && ((1u << r.tpt_log2) < want || (1 << r.tpt_log2) < lanes)) {
+            ++r.tpt_log2;
+        }
+        const size_t at_once = 256u >> r.tpt_log2;
+        blocks               = (tokens + at_once - 1) / at_once;
+        r.chunks             = brief ? (int)((n_vec + 255) / 256) : 1;
+    } else {
+        r.threads = n_vec > 768 && n_vec <= 1152 ? 384 : 256;
+    }
+    const size_t most = (size_t)sms * 8;
+    r.grid            = (unsigned)((blocks < most ? blocks : most) * (size_t)r.chunks);
+    return r;
 }
 
 // dst[r, col0 + c] = e4m3(src[r, c] / scale) for a [rows, cols] source into a matrix with row pitch dst_ld bytes.
@@ -213,27 +267,29 @@ int lyraq_rmsnorm_rope(void* out, const void* qkv, const void* scale, const void
     if ((head_dim != 64 && head_dim != 128) || seq_len > 0x7fffffffu || (dtype != LYRAQ_BF16 && dtype != LYRAQ_F16)) {
         return LYRAQ_ERR_UNSUPPORTED;
     }
-    const size_t   tokens = batch * seq_len;
-    const int      sms    = device_sm_count();
+    const size_t tokens = batch * seq_len;
+    const int    sms    = device_sm_count();
     if (sms <= 0) {
         return LYRAQ_ERR_CUDA;
     }
-    const unsigned grid   = (unsigned)(tokens < (size_t)sms * 8 ? tokens : (size_t)sms * 8);
-    cudaStream_t   s      = (cudaStream_t)stream;
-    cudaError_t    e;
-    if (dtype == LYRAQ_BF16) {
-        using T = __nv_bfloat16;
-        e = (head_dim == 128) ? launch_kernel(rmsnorm_rope_kernel<T, 16>, grid, 256u, (size_t)0, s, 1u, (T*)out, (const T*)qkv,
-                                              (const T*)scale, (const T*)rope, (float)eps, tokens, (int)seq_len, heads)
-                              : launch_kernel(rmsnorm_rope_kernel<T, 8>, grid, 256u, (size_t)0, s, 1u, (T*)out, (const T*)qkv,
-                                              (const T*)scale, (const T*)rope, (float)eps, tokens, (int)seq_len, heads);
-    } else {
-        using T = __half;
-        e = (head_dim == 128) ? launch_kernel(rmsnorm_rope_kernel<T, 16>, grid, 256u, (size_t)0, s, 1u, (T*)out, (const T*)qkv,
-                                              (const T*)scale, (const T*)rope, (float)eps, tokens, (int)seq_len, heads)
-                              : launch_kernel(rmsnorm_rope_kernel<T, 8>, grid, 256u, (size_t)0, s, 1u, (T*)out, (const T*)qkv,
-                                              (const T*)scale, (const T*)rope, (float)eps, tokens, (int)seq_len, heads);
-    }
+    const RopeSplit split = rope_split(tokens, heads, head_dim / 8, out == qkv, sms);
+    cudaStream_t    s     = (cudaStream_t)stream;
+    auto launch = [&](auto* kernel, auto type) {
+        using T = decltype(type);
+        return launch_kernel(kernel, split.grid, split.threads > 0 ? (unsigned)split.threads : 256u, (size_t)0, s, 1u, (T*)out, (const T*)qkv,
+                             (const T*)scale, (const T*)rope, (float)eps, tokens, heads, split.tpt_log2, split.chunks);
+    };
+    auto pick = [&](auto type, auto lanes) {
+        using T             = decltype(type);
+        constexpr int kLanes = decltype(lanes)::value;
+        return split.threads == 0     ? launch(rmsnorm_rope_kernel<T, kLanes, 0>, type)
+               : split.threads == 256 ? launch(rmsnorm_rope_kernel<T, kLanes, 256>, type)
+                                      : launch(rmsnorm_rope_kernel<T, kLanes, 384>, type);
+    };
+    auto pick_lanes = [&](auto type) {
+        return head_dim == 128 ? pick(type, std::integral_constant<int, 16>{}) : pick(type, std::integral_constant<int, 8>{});
+    };
+    const cudaError_t e = dtype == LYRAQ_BF16 ? pick_lanes(__nv_bfloat16{}) : pick_lanes(__half{});
     return cuda_status(e, "cudaLaunchKernelEx(rmsnorm_rope_kernel)");
 }
 

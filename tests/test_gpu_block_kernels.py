@@ -43,6 +43,15 @@ def test_rmsnorm_rope_against_oracle(ops, dtype, batch, seq, heads, head_dim):
     assert_bit_equal(inplace, got, "in place")
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,heads,head_dim", [(6501, 1, 64), (2501, 2, 128), (2501, 8, 128), (1301, 12, 128), (2501, 24, 128), (5, 30, 128),
+                                                   (3, 130, 64), (1190, 33, 128)])
+def test_rmsnorm_rope_threads_of_a_token(ops, dtype, tokens, heads, head_dim):
+    """Every way to deal a token's heads to threads: several tokens to a warp and to a block, a token to a block of either size with more
+    tokens than blocks, a token over several blocks; token counts that fill neither a block nor a round of them.  Bounds as above."""
+    test_rmsnorm_rope_against_oracle(ops, dtype, 1, tokens, heads, head_dim)
+
+
 def test_rmsnorm_rope_with_the_reference_table_fixture(ops):
     """The rotary table of tests/golden/ref_rope_table.npz came out of the reference's own rope / EmbedND; fed to
     lyraq_rmsnorm_rope in that [S, 64, 2, 2] layout (cast to the model type as the reference's wrapper does) the kernel
