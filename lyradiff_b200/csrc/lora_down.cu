@@ -15,10 +15,10 @@
 //   warp 1   MMA issuer; owns the tensor-memory allocation
 //   warps 2-17 (fused form only): the int4 quantize of the same x tiles.  One stage holds, for each of the CTA's 32 rows,
 //            exactly one group of 64 values (a 128-byte row of the swizzled tile), so x is read from memory once for
-//            both results, as in the reference's fused kernel.  A warp takes a whole stage, four rows at a time with eight lanes
-//            to a group (the results of int4_g64_kernel, bit for bit): a lane's eight columns stay the same over the rows, so their
-//            smoothing factors are loaded and inverted once per stage.  A stage goes back to the producer when the MMAs that read it
-//            and its quantizer warp are done.
+//            both results, as in the reference's fused kernel.  A warp takes a whole stage (four share one where K is short), four
+//            rows at a time with eight lanes to a group (the results of int4_g64_kernel, bit for bit): a lane's eight columns stay the
+//            same over the rows, so their smoothing factors are loaded and inverted once per stage.  A stage goes back to the
+//            producer when the MMAs that read it and its quantizer warps are done.
 //
 // The quantizer's arithmetic bounds the fused form, so it has no division in the common case: 36 instructions an element with the
 // IEEE divisions x / smooth, amax / 7 and 1 / s became 20.  Measured, [4608, 12288]: 118 us -> 58; [4608, 3072]: 29 -> 15; [100, 3072]
@@ -151,7 +151,8 @@ __device__ __forceinline__ bool int4_g64_quantize8_fast(const float2 (&x)[R][4],
     return true;
 }
 
-template<bool FUSED, typename T>
+// SHARE quantizer warps take a stage together, its rows dealt out: with fewer stages than warps most of them would have nothing to do.
+template<bool FUSED, int SHARE, typename T>
 __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreads, 1)
 lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_down, const Params p)
 {
@@ -172,7 +173,7 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full_bar(s), 1);
-            mbar_init(empty_bar(s), FUSED ? 2 : 1);   // the MMAs' commit, and the stage's quantizer warp
+            mbar_init(empty_bar(s), FUSED ? 1 + SHARE : 1);   // the MMAs' commit, and the stage's quantizer warps
         }
         mbar_init(done_bar, 1);
         *abort_flag = 0;
@@ -256,9 +257,10 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         const int  sub    = lane >> 3;                // which of a pass's 4 rows
         const bool smooth = p.smooth != nullptr;
         const size_t q_pitch = (size_t)(p.k >> 3), s_pitch = (size_t)(p.k >> 6);
-        uint32_t*    q_out   = p.q + (size_t)(row0 + sub) * q_pitch + part;
-        float*       s_out   = p.q_scale + (size_t)(row0 + sub) * s_pitch;
-        for (int kb = warp - 2; kb < num_kb; kb += kQuantWarps) {
+        const int    r0      = sub + (SHARE > 1 ? 8 * ((warp - 2) % SHARE) : 0);   // this lane's first row of a stage
+        uint32_t*    q_out   = p.q + (size_t)(row0 + r0) * q_pitch + part;
+        float*       s_out   = p.q_scale + (size_t)(row0 + r0) * s_pitch;
+        for (int kb = (warp - 2) / SHARE; kb < num_kb; kb += kQuantWarps / SHARE) {
             const int      stage = kb % kStages;
             const uint32_t phase = (uint32_t)((kb / kStages) & 1);
             float2         ry[4], ns[4];
@@ -283,7 +285,7 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             uint32_t* qrow = q_out + (size_t)kb * 8;
             float*    srow = s_out + kb;
 #pragma unroll 1
-            for (int r = sub; r < kRows; r += 8) {   // this lane's rows r and r + 4: two independent chains
+            for (int r = r0; r < kRows; r += 8 * SHARE) {   // this lane's rows r and r + 4: two independent chains
                 float2 v[2][4];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
@@ -318,8 +320,8 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                         }
                     }
                 }
-                qrow += 8 * q_pitch;
-                srow += 8 * s_pitch;
+                qrow += 8 * SHARE * q_pitch;
+                srow += 8 * SHARE * s_pitch;
             }
             __syncwarp();
             if (lane == 0) {
@@ -331,7 +333,7 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         uint32_t phase = 0;
         const uint32_t idesc = umma_idesc(1u, TypeTag<T>::value == LYRAQ_BF16 ? 1u : 0u, 128, kRows);
         for (int kb = 0; kb < num_kb; ++kb) {
-            if (!mbar_wait_lazy(full_bar(stage), phase, abort_flag)) {
+            if (!(SHARE > 1 ? mbar_wait_warp(full_bar(stage), phase, abort_flag) : mbar_wait_lazy(full_bar(stage), phase, abort_flag))) {
                 give_up(0x2200u | (unsigned)stage);
                 break;
             }
@@ -363,15 +365,15 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     }
 }
 
-template<bool FUSED, typename T> static int launch(unsigned grid, const CUtensorMap& tx, const CUtensorMap& td, const Params& p, cudaStream_t stream)
+template<bool FUSED, int SHARE, typename T> static int launch(unsigned grid, const CUtensorMap& tx, const CUtensorMap& td, const Params& p, cudaStream_t stream)
 {
     static bool smem_raised[64] = {};
-    const int   st = raise_dynamic_smem_once(lora_down_kernel<FUSED, T>, (int)kSmemTotal, smem_raised,
+    const int   st = raise_dynamic_smem_once(lora_down_kernel<FUSED, SHARE, T>, (int)kSmemTotal, smem_raised,
                                            "cudaFuncSetAttribute(lora_down_kernel, dynamic shared memory)");
     if (st != LYRAQ_OK) {
         return st;
     }
-    return cuda_status(launch_kernel(lora_down_kernel<FUSED, T>, grid, (unsigned)(FUSED ? kThreadsFused : kThreads), (size_t)kSmemTotal, stream, 1u,
+    return cuda_status(launch_kernel(lora_down_kernel<FUSED, SHARE, T>, grid, (unsigned)(FUSED ? kThreadsFused : kThreads), (size_t)kSmemTotal, stream, 1u,
                                      tx, td, p),
                        "cudaLaunchKernelEx(lora_down_kernel)");
 }
@@ -422,8 +424,15 @@ static int launch_lora_down_impl(float* act, const void* x, const void* down, in
     }
     const unsigned grid = (unsigned)((m + lora::kRows - 1) / lora::kRows);
     const bool bf16 = dtype == LYRAQ_BF16;
-    return fused ? (bf16 ? lora::launch<true, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<true, __half>(grid, tx, td, p, stream))
-                 : (bf16 ? lora::launch<false, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<false, __half>(grid, tx, td, p, stream));
+    if (!fused) {
+        return bf16 ? lora::launch<false, 1, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<false, 1, __half>(grid, tx, td, p, stream);
+    }
+    // Up to half as many stages as quantizer warps: four warps to a stage, and an issuer that polls without pauses.  With a warp to a stage
+    // [4608, 64] took 4.4 us, so 2.9; [512, 128] 4.3 / 2.9; [4608, 512] 5.4 / 5.1.
+    if (k <= 64 * lora::kQuantWarps / 2) {
+        return bf16 ? lora::launch<true, 4, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<true, 4, __half>(grid, tx, td, p, stream);
+    }
+    return bf16 ? lora::launch<true, 1, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<true, 1, __half>(grid, tx, td, p, stream);
 }
 
 int launch_lora_down(float* act, const void* x, const void* down, int dtype, size_t m, size_t k, cudaStream_t stream)

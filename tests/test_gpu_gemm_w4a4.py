@@ -167,6 +167,14 @@ def test_lora_down_next_to_the_quantize(ops, m, k, dt):
 
 
 @pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m", [1, 31, 700])
+@pytest.mark.parametrize("k", [128, 256, 448, 512, 576])
+def test_lora_down_with_few_stages(ops, m, k, dt):
+    """Up to 512 columns four quantizer warps share a stage, a group of 64 columns; from there each takes its own.  Bounds as above."""
+    test_lora_down_next_to_the_quantize(ops, m, k, dt)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("m,k", [(1, 64), (33, 1600), (700, 3072)])
 @pytest.mark.parametrize("case", ["plain", "no smooth", "wide smooth", "far smooth", "wide x", "not finite", "ties"])
 def test_quantize_beside_the_low_rank_product_has_the_divisions_bits(ops, m, k, dt, case):
