@@ -413,6 +413,10 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
         const int    quadrant = warp & 3;
         const float* sums     = reinterpret_cast<const float*>(gen_base + kSumOffset);
+        // Read once, ahead of the work: behind each block's waits the load and the division took 0.6 of 256 tokens' 9.65 us.  A scale that
+        // belongs to no row is not read (out_scale[1] may be null).
+        const float  qs0      = p.out_e4m3 && p.split > 0 ? 1.0f / ld_f32(p.out_scale[0]) : 1.0f;
+        const float  qs1      = p.out_e4m3 && p.split < p.seq ? 1.0f / ld_f32(p.out_scale[1]) : 1.0f;
         bool         ok       = true;
         int          done     = 0;
         for (int blk = blockIdx.x; ok && blk < p.blocks; blk += gridDim.x, ++done) {
@@ -421,6 +425,9 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
             const int b  = blk / (p.q_blocks * p.heads);
 #pragma unroll 1
             for (int t = 0; t < kQTiles; ++t) {
+                const int       row   = q0 + t * kTile + quadrant * 32 + lane;   // row inside the sequence
+                const int       part  = row >= p.split ? 1 : 0;
+                const long long r_out = part ? row - p.split : row;
                 if (!mbar_wait_lazy(l_full(t), (uint32_t)(done & 1), abort_flag, p.wait_limit_ns) ||
                     !mbar_wait_warp(o_full(t), (uint32_t)(done & 1), abort_flag, p.wait_limit_ns)) {
                     give_up(0x3320u | (unsigned)t);
@@ -428,16 +435,15 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
                     break;
                 }
                 tc_fence_after_sync();
-                const int       row   = q0 + t * kTile + quadrant * 32 + lane;   // row inside the sequence
-                const int       part  = row >= p.split ? 1 : 0;
-                const long long r_out = part ? row - p.split : row;
-                const float     inv_l = 1.0f / sums[t * kTile + quadrant * 32 + lane];
-                // rows past the end of the sequence belong to no part (out_scale[1] may be null): they load nothing, store nothing
-                const float     qs     = (p.out_e4m3 && row < p.seq) ? 1.0f / ld_f32(p.out_scale[part]) : 1.0f;
+                const float     inv_l  = 1.0f / sums[t * kTile + quadrant * 32 + lane];
+                const float     qs     = part ? qs1 : qs0;
                 const uint32_t  o_addr = tmem_base + ((uint32_t)(quadrant * 32) << 16) + (uint32_t)(256 + t * 128);
                 uint8_t*        dst    = static_cast<uint8_t*>(p.out[part]) +
                                ((long long)b * p.out_batch[part] + r_out * p.out_ld[part] + (long long)h * kHeadDim) * (p.out_e4m3 ? 1 : 2);
-                auto value = [&](uint32_t lo, uint32_t hi) { return Pair<T>::from_f32(__uint_as_float(lo) * inv_l, __uint_as_float(hi) * inv_l); };
+                auto value = [&](uint32_t lo, uint32_t hi) {
+                    const float2 v = mul_f32x2(make_float2(__uint_as_float(lo), __uint_as_float(hi)), make_float2(inv_l, inv_l));
+                    return Pair<T>::from_f32(v.x, v.y);
+                };
                 // the whole row is read before the first store: the accumulator and the sums may be overwritten while the rows go out
                 auto release = [&]() {
                     tc_fence_before_sync();
@@ -447,7 +453,9 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
                         mbar_arrive(l_empty(t));
                     }
                 };
-                if (p.out_e4m3) {
+                if (q0 + t * kTile >= p.seq) {
+                    release();   // a tile without rows: converting it all the same took 64 tokens 0.4 of 6.5 us
+                } else if (p.out_e4m3) {
                     uint32_t w[32];
 #pragma unroll
                     for (int cc = 0; cc < 4; ++cc) {
@@ -456,8 +464,10 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_qkv, const __grid_
                         tmem_ld_wait();
 #pragma unroll
                         for (int k = 0; k < 8; ++k) {
-                            const float2 x = Pair<T>::to_f32(value(o[4 * k], o[4 * k + 1])), y = Pair<T>::to_f32(value(o[4 * k + 2], o[4 * k + 3]));
-                            w[cc * 8 + k]  = f32x2_to_e4m3x2(x.x * qs, x.y * qs) | (f32x2_to_e4m3x2(y.x * qs, y.y * qs) << 16);
+                            const float2 q2 = make_float2(qs, qs);
+                            const float2 x  = mul_f32x2(Pair<T>::to_f32(value(o[4 * k], o[4 * k + 1])), q2);
+                            const float2 y  = mul_f32x2(Pair<T>::to_f32(value(o[4 * k + 2], o[4 * k + 3])), q2);
+                            w[cc * 8 + k]   = f32x2_to_e4m3x2(x.x, x.y) | (f32x2_to_e4m3x2(y.x, y.y) << 16);
                         }
                     }
                     release();

@@ -181,6 +181,30 @@ def test_attention_e4m3_output_into_a_column_window_and_split(ops):
     assert_bit_equal(b16, r[:, split:].reshape(-1, width), "image part 16-bit")
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch,seq,split", [(3, 1, 1), (60, 64, 64), (2, 128, 0), (1, 129, 128), (2, 300, 299), (90, 257, 100)])
+def test_attention_e4m3_of_short_sequences(ops, dtype, batch, seq, split):
+    """Blocks whose second tile of 128 rows has none, one or some, alone and several to a CTA, with one and two outputs (an output without
+    rows needs no scale that can be read): the e4m3 codes of the 16-bit result."""
+    g = torch.Generator().manual_seed(batch + seq)
+    width = 3 * 128
+    qkv = cu(_qkv(batch, seq, 3, 128, dtype, g))
+    ref = torch.empty(batch * seq, width, dtype=dtype, device="cuda")
+    ops.flash_attention(qkv, batch, seq, 3, 128, out=ref)
+    r = ref.cpu().reshape(batch, seq, width)
+    scales = [torch.tensor([0.02], device="cuda"), torch.tensor([0.013], device="cuda")]
+    a, b = (torch.full((batch * n + 1, width), 0x55, dtype=torch.uint8, device="cuda") for n in (split, seq - split))
+    if split == seq:
+        ops.flash_attention(qkv, batch, seq, 3, 128, out=a[:-1], out_scale=scales[0])
+    else:
+        ops.flash_attention(qkv, batch, seq, 3, 128, out=a[:batch * split] if split else a, out_scale=scales[0], out2=b[:-1], out2_scale=scales[1],
+                            split=split)
+    check_status()
+    assert_bit_equal(a[:-1], quant.fp8_quant(r[:, :split].reshape(-1, width), scales[0].cpu()), "first rows")
+    assert_bit_equal(b[:-1], quant.fp8_quant(r[:, split:].reshape(-1, width), scales[1].cpu()), "other rows")
+    assert bool((a[-1] == 0x55).all()) and bool((b[-1] == 0x55).all())
+
+
 def test_attention_flux_size_sample_and_properties(ops):
     """4608 tokens, 24 heads (the FLUX.1-dev shape): a strided sample of query rows against the oracle (which needs all
     keys but only the sampled queries), run-to-run identical bits, and the convexity property: every output lies inside
