@@ -362,7 +362,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint32_t*      tmem_slot  = reinterpret_cast<uint32_t*>(gen_base + S::kBarOffset + 8 * (2 * kStages + 4));
     volatile int*  abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int      warp    = warp_index();
+    // A pair's warp index stays a per-lane value: as a uniform one it made each tile of the INT8 epilogue 2.8 us longer (same
+    // registers, no spills).  Forced pairs, [8192, 5120, 640] 41.4 us / 66.7 uniform, [16384, 1280, 2048] 32.4 / 43.4, [2048, 1280, 5120] 19.1 / 21.9,
+    // FP8 level; one CTA with 128 columns gains up to 5 % by it.
+    const int      warp    = CTAS == 2 ? (int)(threadIdx.x >> 5) : warp_index();
     const int      lane    = threadIdx.x & 31;
     const uint32_t rank    = (CTAS == 2) ? cluster_ctarank() : 0u;  // position in the pair; 0 = leader
     const bool     leader  = (rank == 0);
