@@ -170,6 +170,12 @@ __device__ __forceinline__ float ld_f32(const float* p)
     asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ uint32_t ld_u16(const void* p)
+{
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ float4 ld_f32x4(const float4* p)
 {
     float4 v;
