@@ -291,6 +291,35 @@ def test_wide_kernel_gives_the_same_bits_as_the_one_without_workspace(ops, force
             assert not bool((ample[:n * k] == 0xA5).any())      # it was the wide kernel: no e4m3 code of -8 .. 7 is 0xA5
 
 
+@pytest.mark.parametrize("k", [64, 192, 576, 768, 1088])
+@pytest.mark.parametrize("dt,sb_dtype", [(torch.bfloat16, torch.float16), (torch.float16, torch.float32)])
+def test_wide_kernel_tiles_that_start_anywhere_in_the_rings(ops, forced_wide, k, dt, sb_dtype):
+    """More tiles than SMs with an odd number of scale slots a tile, the last one full or part filled, by both scale loaders: a CTA's
+    second and third tile start in the other slot, the other raw buffer and the other parity of each."""
+    test_wide_kernel_gives_the_same_bits_as_the_one_without_workspace(ops, forced_wide, 4099, 1544, k, dt, sb_dtype)
+
+
+@pytest.mark.parametrize("k", [256, 512, 768])
+@pytest.mark.parametrize("sb_dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("off_a,off_b", [(1, 0), (0, 1), (1, 1), (4, 8)])
+def test_wide_kernel_with_scales_off_their_alignment(ops, forced_wide, k, sb_dtype, off_a, off_b):
+    """Group counts that TMA could fetch in arrays that do not start on 16 bytes (the last pair of offsets does): the same bits."""
+    m, n, G = 300, 264, k // 64
+    g = torch.Generator(device="cuda").manual_seed(k + off_a)
+    a, b = (torch.randint(0, 256, (r, k // 2), generator=g, device="cuda", dtype=torch.uint8) for r in (m, n))
+    sa, sb = torch.rand(m * G + off_a, generator=g, device="cuda"), torch.rand(n * G + off_b, generator=g, device="cuda").to(sb_dtype)
+    out = []
+    for sa2, sb2, ws in ((sa[off_a:].view(m, G), sb[off_b:].view(n, G), _wide_bytes(m, n, k)),
+                         (sa[off_a:].clone().view(m, G), sb[off_b:].clone().view(n, G), 0)):
+        d = torch.full((m, n), -1.0, dtype=torch.bfloat16, device="cuda")
+        arena = torch.full((ws,), 0xA5, dtype=torch.uint8, device="cuda")
+        ops.invoke_fused_w4a4_gemm_and_lora_up(d, a, b, None, None, sa2, sb2, workspace=arena)
+        check_status()
+        assert not bool((arena[:n * k] == 0xA5).any())
+        out.append(d.cpu())
+    assert_bit_equal(out[0], out[1])
+
+
 def test_wide_kernel_workspace_is_optional_and_its_size_is_checked(ops, forced_wide):
     from lyradiff_b200 import _lib
     L = _lib.lib()
