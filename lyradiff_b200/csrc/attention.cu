@@ -82,7 +82,7 @@ struct Params {
     const float*  out_scale[2];  // e4m3 output: per-tensor scale of each part (1 / scale applied); unused otherwise
     int           out_e4m3;
     int           split;
-    int           batch, seq, heads;
+    int           seq, heads;
     int           q_blocks;      // ceil(seq / 256)
     int           blocks;        // batch * heads * q_blocks
     float         scale_log2;    // softmax scale * log2(e)
@@ -721,7 +721,6 @@ int launch_attention(void* out, int out_dtype, size_t out_ld, const float* out_s
     p.out_scale[1] = out2_scale;
     p.out_e4m3     = e4m3 ? 1 : 0;
     p.split        = (int)split;
-    p.batch        = (int)batch;
     p.seq          = (int)seq;
     p.heads        = heads;
     p.q_blocks     = (int)((seq + attn::kQTiles * attn::kTile - 1) / (attn::kQTiles * attn::kTile));

@@ -1,4 +1,5 @@
-// Low-rank down projection of the W4A4 linear: act[m, 32] = x[m, k] * lora_down[32, k]^T, 16-bit inputs, fp32 out.
+// Low-rank down projection of the W4A4 linear, act[m, 32] = x[m, k] * lora_down[32, k]^T (16-bit inputs, fp32 out), and in the same
+// launch the int4 quantize of x.
 //
 // The reference computes this inside its int4 quantize kernel with one mma.sync tile per 64 columns and a
 // floating-point atomic add per tile (src/lyradiff/kernels/w4a4_gemm/w4a4_gemm.cu:769-954), so the order of the 48
@@ -7,20 +8,20 @@
 //
 // The product is formed transposed, D[r, j] = sum_k lora_down[r, k] * x[row0 + j, k]: tcgen05.mma needs M >= 64, and
 // with the 32 rows of x on the N side 4608 tokens give 144 CTAs (one per SM) instead of 36.  The M side is the 32 rows
-// of lora_down; the 96 rows behind them are whatever lies next in shared memory, which only reaches accumulator lanes that
-// nobody reads.
+// of lora_down; the 96 rows behind them are whatever lies next in shared memory: the tiles of other stages, which the TMA
+// may be writing while the MMA reads them.  They only reach accumulator lanes that nobody reads.
 //
 //   warp 0   TMA producer (lora_down tile and x tile, 32 rows x 128 B each, ring of 24 stages);
 //            afterwards it reads accumulator lanes 0..31 and stores act
 //   warp 1   MMA issuer; owns the tensor-memory allocation
-//   warps 2-17 (fused form only): the int4 quantize of the same x tiles.  One stage holds, for each of the CTA's 32 rows,
+//   warps 2-17  the int4 quantize of the same x tiles.  One stage holds, for each of the CTA's 32 rows,
 //            exactly one group of 64 values (a 128-byte row of the swizzled tile), so x is read from memory once for
 //            both results, as in the reference's fused kernel.  A warp takes a whole stage (four share one where K is short), four
 //            rows at a time with eight lanes to a group (the results of int4_g64_kernel, bit for bit): a lane's eight columns stay the
 //            same over the rows, so their smoothing factors are loaded and inverted once per stage.  A stage goes back to the
 //            producer when the MMAs that read it and its quantizer warps are done.
 //
-// The quantizer's arithmetic bounds the fused form, so it has no division in the common case: 36 instructions an element with the
+// The quantizer's arithmetic bounds the kernel, so it has no division in the common case: 36 instructions an element with the
 // IEEE divisions x / smooth, amax / 7 and 1 / s became 20.  Measured, [4608, 12288]: 118 us -> 58; [4608, 3072]: 29 -> 15; [100, 3072]
 // f16: 80 -> under 18.
 // All waits are bounded; a timeout sets the status word and the block leaves.
@@ -45,15 +46,13 @@ constexpr int kXOffset   = kStages * kTile;       // all lora_down tiles, then a
 static_assert(kXOffset >= 128 * kBlockKB, "");    // the last lora_down tile stay inside the allocation
 constexpr int kBarOffset = 2 * kStages * kTile;
 constexpr int kSmemTotal = kBarOffset + 512 + 1024;
-constexpr int kThreads   = 64;                    // down projection alone
 constexpr int kQuantWarps = 16;
-constexpr int kThreadsFused = kThreads + 32 * kQuantWarps;
+constexpr int kThreads   = 64 + 32 * kQuantWarps;
 
 struct Params {
     float*        act;   // [m, 32]
     int           m, k;
     unsigned int* status;
-    // fused int4 quantize (all null / 0 for the down projection alone)
     uint32_t*     q;        // [m, k / 8]: eight nibbles per word
     float*        q_scale;  // [m, k / 64]
     const float*  smooth;   // [k] or null
@@ -152,8 +151,8 @@ __device__ __forceinline__ bool int4_g64_quantize8_fast(const float2 (&x)[R][4],
 }
 
 // SHARE quantizer warps take a stage together, its rows dealt out: with fewer stages than warps most of them would have nothing to do.
-template<bool FUSED, int SHARE, typename T>
-__global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreads, 1)
+template<int SHARE, typename T>
+__global__ void __launch_bounds__(kThreads, 1)
 lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_down, const Params p)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -173,7 +172,7 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(full_bar(s), 1);
-            mbar_init(empty_bar(s), FUSED ? 1 + SHARE : 1);   // the MMAs' commit, and the stage's quantizer warps
+            mbar_init(empty_bar(s), 1 + SHARE);   // the MMAs' commit, and the stage's quantizer warps
         }
         mbar_init(done_bar, 1);
         *abort_flag = 0;
@@ -251,7 +250,7 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         } else if (lane == 0) {
             report_timeout(p.status, 0x2300u);
         }
-    } else if (FUSED && warp >= 2) {
+    } else if (warp >= 2) {
         // ------------------------------------------------------------------ int4 quantize of the staged x tiles
         const int  part   = lane & 7;                 // which 8 values of the group of 64
         const int  sub    = lane >> 3;                // which of a pass's 4 rows
@@ -365,28 +364,28 @@ lora_down_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     }
 }
 
-template<bool FUSED, int SHARE, typename T> static int launch(unsigned grid, const CUtensorMap& tx, const CUtensorMap& td, const Params& p, cudaStream_t stream)
+template<int SHARE, typename T> static int launch(unsigned grid, const CUtensorMap& tx, const CUtensorMap& td, const Params& p, cudaStream_t stream)
 {
     static bool smem_raised[64] = {};
-    const int   st = raise_dynamic_smem_once(lora_down_kernel<FUSED, SHARE, T>, (int)kSmemTotal, smem_raised,
+    const int   st = raise_dynamic_smem_once(lora_down_kernel<SHARE, T>, (int)kSmemTotal, smem_raised,
                                            "cudaFuncSetAttribute(lora_down_kernel, dynamic shared memory)");
     if (st != LYRAQ_OK) {
         return st;
     }
-    return cuda_status(launch_kernel(lora_down_kernel<FUSED, SHARE, T>, grid, (unsigned)(FUSED ? kThreadsFused : kThreads), (size_t)kSmemTotal, stream, 1u,
+    return cuda_status(launch_kernel(lora_down_kernel<SHARE, T>, grid, (unsigned)kThreads, (size_t)kSmemTotal, stream, 1u,
                                      tx, td, p),
                        "cudaLaunchKernelEx(lora_down_kernel)");
 }
 
 }  // namespace lora
 
-// act[m, 32] (fp32) = x[m, k] * down[32, k]^T; x and down of the same 16-bit type; k a multiple of 8.  With q != null the
-// same launch also writes the int4 group-64 quantization of x / smooth (packed nibbles q [m, k / 2 bytes], fp32 scales
-// q_scale [m, k / 64]); k then has to be a multiple of 64.
-static int launch_lora_down_impl(float* act, const void* x, const void* down, int dtype, size_t m, size_t k, uint8_t* q, float* q_scale,
-                                 const float* smooth, cudaStream_t stream)
+// The reference's fused_quantized_and_lora_down_simple (w4a4_gemm.cu:769-954) as ONE launch over one read of x: the int4 group-64
+// quantization of x / smooth (packed nibbles q [m, k / 2 bytes], fp32 scales q_scale [m, k / 64]) and act[m, 32] (fp32) =
+// x[m, k] * down[32, k]^T; x and down of the same 16-bit type, k a multiple of 64.
+int launch_quant_int4_lora_down(uint8_t* q, float* q_scale, float* act, const void* x, const void* down, const float* smooth, int dtype,
+                                size_t m, size_t k, cudaStream_t stream)
 {
-    if (act == nullptr || x == nullptr || down == nullptr) {
+    if (q == nullptr || act == nullptr || x == nullptr || down == nullptr) {
         return LYRAQ_ERR_INVALID_ARG;
     }
     if (dtype != LYRAQ_BF16 && dtype != LYRAQ_F16) {
@@ -395,11 +394,10 @@ static int launch_lora_down_impl(float* act, const void* x, const void* down, in
     if (!aligned16(x) || !aligned16(down) || (reinterpret_cast<uintptr_t>(act) & 3u) != 0) {
         return LYRAQ_ERR_INVALID_ARG;
     }
-    const bool fused = q != nullptr;
-    if (fused && (q_scale == nullptr || (reinterpret_cast<uintptr_t>(q) & 3u) != 0 || (smooth != nullptr && !aligned16(smooth)))) {
+    if (q_scale == nullptr || (reinterpret_cast<uintptr_t>(q) & 3u) != 0 || (smooth != nullptr && !aligned16(smooth))) {
         return LYRAQ_ERR_INVALID_ARG;
     }
-    if ((k & 7) != 0 || k == 0 || k > 0x3fffffffu || m > 0x7fffffffu || (fused && (k & 63) != 0)) {
+    if ((k & 63) != 0 || k == 0 || k > 0x3fffffffu || m > 0x7fffffffu) {
         return LYRAQ_ERR_UNSUPPORTED;
     }
     lora::Params p{};
@@ -424,30 +422,12 @@ static int launch_lora_down_impl(float* act, const void* x, const void* down, in
     }
     const unsigned grid = (unsigned)((m + lora::kRows - 1) / lora::kRows);
     const bool bf16 = dtype == LYRAQ_BF16;
-    if (!fused) {
-        return bf16 ? lora::launch<false, 1, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<false, 1, __half>(grid, tx, td, p, stream);
-    }
     // Up to half as many stages as quantizer warps: four warps to a stage, and an issuer that polls without pauses.  With a warp to a stage
     // [4608, 64] took 4.4 us, so 2.9; [512, 128] 4.3 / 2.9; [4608, 512] 5.4 / 5.1.
     if (k <= 64 * lora::kQuantWarps / 2) {
-        return bf16 ? lora::launch<true, 4, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<true, 4, __half>(grid, tx, td, p, stream);
+        return bf16 ? lora::launch<4, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<4, __half>(grid, tx, td, p, stream);
     }
-    return bf16 ? lora::launch<true, 1, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<true, 1, __half>(grid, tx, td, p, stream);
-}
-
-int launch_lora_down(float* act, const void* x, const void* down, int dtype, size_t m, size_t k, cudaStream_t stream)
-{
-    return launch_lora_down_impl(act, x, down, dtype, m, k, nullptr, nullptr, nullptr, stream);
-}
-
-// The reference's fused_quantized_and_lora_down_simple (w4a4_gemm.cu:769-954) as ONE launch over one read of x.
-int launch_quant_int4_lora_down(uint8_t* q, float* q_scale, float* act, const void* x, const void* down, const float* smooth, int dtype,
-                                size_t m, size_t k, cudaStream_t stream)
-{
-    if (q == nullptr) {
-        return LYRAQ_ERR_INVALID_ARG;
-    }
-    return launch_lora_down_impl(act, x, down, dtype, m, k, q, q_scale, smooth, stream);
+    return bf16 ? lora::launch<1, __nv_bfloat16>(grid, tx, td, p, stream) : lora::launch<1, __half>(grid, tx, td, p, stream);
 }
 
 }  // namespace lyraq

@@ -11,7 +11,6 @@ namespace lyraq {
 
 int device_sm_count();  // gemm_dense.cu
 unsigned int* status_word_ptr();  // api.cu
-int launch_lora_down(float* act, const void* x, const void* down, int dtype, size_t m, size_t k, cudaStream_t stream);
 int launch_quant_int4_lora_down(uint8_t* q, float* q_scale, float* act, const void* x, const void* down, const float* smooth, int dtype,
                                 size_t m, size_t k, cudaStream_t stream);  // lora_down.cu
 
