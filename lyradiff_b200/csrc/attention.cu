@@ -32,7 +32,7 @@
 // bound by shared memory), the next block's start and the last one's epilogue out of the way of the softmax, and above all an issuer
 // whose code between two MMAs is short: whole-warp waits of a few instructions (see mbar_wait_warp) and no slow path in between.
 // Not kept: exponentials started from the old maximum with the new one found beside them (the same time), two softmax warps per
-// 32 rows (3 % fewer clocks, the same time at the power limit), P handed over in parts of 96 + 32 keys (3 % slower), a quarter of the exponentials on the FMA
+// 32 rows (3 % fewer clocks, the same time at the power limit), P handed over in parts of 96 + 32 keys (3 to 4 % slower), a quarter of the exponentials on the FMA
 // pipe (2 % slower than an eighth).
 #include "common.cuh"
 #include "sm100_ptx.cuh"

@@ -1136,6 +1136,11 @@ int device_sm_count()
 // Tile choice.  Cost of a configuration = waves (tiles / units that run at once) x work per tile.  A CTA pair with a
 // 256 x 256 tile moves a third less operand traffic per flop than a single CTA with 128 x 256, so it is preferred
 // (10 % bonus) whenever its wave quantisation is not worse; small or narrow problems fall back to one CTA.
+// Both numbers below, 2048 and 0.9, were set when a pass over a barrier cost a pair more than it does now.  At the FLUX and SDXL shapes the
+// choice is still the fastest one (FP8 [4608, 9216, 3072] pair 89 us, one CTA 101, 128 columns 115; INT8 [8192, 640, 2560] 128 columns 15.8,
+// one CTA 17.3, pair 17.8) but not everywhere: one round of pairs is 9 to 23 % slower than one round of single CTAs (FP8 [1317, 3072, 3072]
+// 15.6 / 12.7, [512, 9216, 3072] 16.0 / 13.0), and 128 columns that save rounds lose to the pair at K = 12288 ([2829, 5120, 12288]
+// 195 / 163) and to one CTA at K = 640 (INT8 [6249, 10240, 640] 64 / 46).
 struct TileChoice {
     int block_n;
     int ctas;
@@ -1219,11 +1224,13 @@ static int g_forced_tile = 0;
 
 // Whether the few-token kernel (gemm_skinny.cu) takes an FP8 problem: a plain epilogue, and so few rows that it is the faster one.
 // Its time grows by 0.1 to 0.25 us a row where the dense kernel's does not grow at all, and what it gains at one row grows with K and,
-// for small K, with the tiles.  Dense against few-token, us: 4 rows of [256, 256] 3.8 / 3.4, 8 rows 3.9 / 4.4, 16 rows 3.9 / 6.2; 6 rows
-// of [12288, 256] 4.9 / 4.4, 10 rows 4.8 / 5.3; 6 rows of [1280, 1024] 5.3 / 5.2, 16 rows 5.3 / 6.3; 12 rows of [3072, 1536] 7.0 / 7.1;
-// 16 rows of [3072, 1664] 7.7 / 7.5 and of [1280, 2048] 6.9 / 5.7.  From 16 K blocks on all 16 rows gain, except that the dense kernel
+// for small K, with the tiles.  Dense against few-token, us: 4 rows of [256, 256] 4.2 / 4.0, 8 rows 4.2 / 5.0; 6 rows of [12288, 256]
+// 5.3 / 5.0, 10 rows 5.3 / 6.0; 6 rows of [1280, 1024] 5.7 / 5.8, 16 rows 5.7 / 7.0; 12 rows of [3072, 1536] 6.5 / 7.0; 16 rows of
+// [3072, 1664] 6.8 / 7.4 and of [1280, 2048] 7.1 / 6.3.  From 16 K blocks on all 16 rows gain, except that the dense kernel
 // gets 1.4 times faster once X has 128 KB, which with more tiles than four CTAs along K can share is enough for it to win:
-// [12, 12288, 8192] 37.4 / 24.9, [16, 12288, 8192] 23.2 / 25.4.
+// [12, 12288, 8192] 35.7 / 25.7, [16, 12288, 8192] 24.1 / 25.7.  On 196 of 203 pairs (1 to 16 rows, n 256 .. 18432, k 256 .. 12288) the
+// choice is the faster kernel or within 2 % of it; the line was drawn when the dense kernel's waits took longer, and the other seven, 12 to 16
+// rows at 12 and 13 K blocks above all, are 4 to 9 % slower by it.
 static bool few_tokens(const GemmParams& p)
 {
     if (p.M > kSkinnyRows || p.epi.gate != nullptr || p.epi.rope != nullptr || p.epi.out_q_scale != nullptr || p.epi.ldc != p.N) {

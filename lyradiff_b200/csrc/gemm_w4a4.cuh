@@ -30,14 +30,15 @@ struct Params {
 
 constexpr int kLoraRank = 32;
 
-// Whether the wide path is the faster one, in microseconds of each kernel.  A wave of gemm_w4a4_kernel's 128 x 128 tiles over all SMs
+// Whether the wide path is the faster one, by what a wave of each kernel costs in microseconds.  A wave of gemm_w4a4_kernel's 128 x 128 tiles over all SMs
 // takes 3.4 + 7.4 (k / 1024), one of the wide kernel's 256 x 128 tiles 7.2 + 10.3 (k / 1024); fp32 rows leave the wide kernel element
 // by element, which adds 26 to a wave.  The rewrite moves 1.5 bytes per element of both operands at 5 TB/s behind a launch of 4.
-// (Both kernels have become faster by about the same share since, 10 to 14 %; the line was left where it lies.)
-// Fitted to 273 measured pairs, m 64 .. 8192, n 3072 .. 21504, k 64 .. 12288: on none of them is the choice more than 2 % slower than
-// the other one.  16-bit outputs: [4608, 12288, 3072] 24 waves 616 us against 12 waves 477; [1024, 12288, 3072] 6 / 3 waves 159 / 137;
-// [2048, 3072, 3072] 3 / 2 waves 84 / 88; [8192, 3072, 512] 11 / 6 waves 80 / 83.  fp32: [4608, 12288, 3072] 655 / 837,
-// [4608, 3072, 12288] 574 / 522.
+// The constants were fitted to 273 pairs, m 64 .. 8192, n 3072 .. 21504, k 64 .. 12288.  Both kernels have become faster since, the wide
+// one more (14 % against 5 at [4608, 12288, 3072]), so the times above are too long for both and the line lies too far on the
+// narrow side.  Both timed again at 269 pairs that lie within a third of it, with either loader of the scales: where it says wide, wide
+// was the faster one (within 2 %); of those where it says narrow, 28 would have been 2 to 13 % faster wide.  Now, narrow / wide, us:
+// [4608, 12288, 3072] 582 / 412; [1024, 12288, 3072] 152 / 119; [2048, 3072, 3072] 79 / 75 and [8192, 3072, 512] 79 / 72, both of which go
+// narrow; [8192, 12288, 128] 190 / 167 likewise.  fp32: [4608, 12288, 3072] 625 / 766, [4608, 3072, 12288] 542 / 466.
 inline bool wide_pays(size_t m, size_t n, size_t k, int sms, bool fp32_out)
 {
     const size_t u      = sms > 0 ? (size_t)sms : 148;

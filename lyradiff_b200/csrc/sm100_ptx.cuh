@@ -26,8 +26,8 @@ __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (i
 // True in one lane of the (whole, converged) warp, always the same one.  A role run by one thread enters its branch through this
 // and not through `lane == 0`: the tcgen05 and TMA instructions take their operands from registers that belong to the warp, and
 // only behind elect.sync does the compiler know that a single lane is active.  Behind a lane test an issuer started one tcgen05.mma
-// per 65 clocks whatever its size.  Measured with this alone: attention at 4608 x 24 x 128 250 -> 223 us, INT8 GEMM
-// [8192, 5120, 640] 38.1 -> 36.1, W4A4 GEMM [4608, 12288, 3072] 484 -> 460, FP8 GEMM [4608, 9216, 3072] 96.1 -> 94.9.
+// per 65 clocks whatever its size.  Measured with this alone: attention at 4608 x 24 x 128 250 -> 221 us, FP8 single-stream block at 4608
+// tokens 820 -> 779, W4A4 linear [4608, 12288, 3072] 528 -> 522; single FP8 and INT8 linears the same within their spread.
 __device__ __forceinline__ bool elect_one()
 {
     uint32_t one;
