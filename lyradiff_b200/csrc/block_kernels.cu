@@ -23,7 +23,7 @@ int device_sm_count();  // gemm_dense.cu
 //
 // THREADS > 0: a block of THREADS takes a token at a time.  THREADS = 0: a block of 256 has 2^tpt_log2 threads to a token, several tokens at
 // a time where that leaves room, and `chunks` blocks share a token.
-template<typename T, int LANES, int THREADS>
+template<typename T, int LANES, int THREADS, int FLIGHT>
 __global__ void __launch_bounds__(THREADS > 0 ? THREADS : 256) rmsnorm_rope_kernel(T* out, const T* qkv, const T* scale, const T* rope,
                                                                                    float eps, size_t tokens, int heads, int tpt_log2, int chunks)
 {
@@ -31,7 +31,6 @@ __global__ void __launch_bounds__(THREADS > 0 ? THREADS : 256) rmsnorm_rope_kern
     grid_launch_dependents();
     grid_dependency_wait();
     constexpr int kHeadDim = LANES * 8;
-    constexpr int kFlight  = 3;
     const int     part     = threadIdx.x % LANES;                    // which 8 elements of a head
     const int     n_q      = heads * LANES, n_qk = 2 * n_q;          // vectors of the q heads, of the q and k heads
     const int     n_vec    = out == qkv ? n_qk : 3 * n_q;            // the v heads are copied unless they are in place
@@ -41,8 +40,9 @@ __global__ void __launch_bounds__(THREADS > 0 ? THREADS : 256) rmsnorm_rope_kern
     constexpr bool kSplit  = THREADS == 0;
     const int     tpt      = kSplit ? 1 << tpt_log2 : THREADS;
     const int     mine     = kSplit ? (int)threadIdx.x & (tpt - 1) : (int)threadIdx.x;
-    const unsigned blk     = kSplit ? blockIdx.x / (unsigned)chunks : blockIdx.x, blks = kSplit ? gridDim.x / (unsigned)chunks : gridDim.x;
-    const int     first    = (kSplit ? (int)(blockIdx.x - blk * (unsigned)chunks) * tpt : 0) + mine;    // of the token's vectors
+    const bool    shared   = kSplit && chunks > 1;                  // (spares other calls the division)
+    const unsigned blk     = shared ? blockIdx.x / (unsigned)chunks : blockIdx.x, blks = shared ? gridDim.x / (unsigned)chunks : gridDim.x;
+    const int     first    = (shared ? (int)(blockIdx.x - blk * (unsigned)chunks) * tpt : 0) + mine;    // of the token's vectors
     const int     step     = kSplit ? tpt * chunks : THREADS;
     const size_t  sub      = kSplit ? threadIdx.x >> tpt_log2 : 0;
     const size_t  at_once  = kSplit ? 256u >> tpt_log2 : 1;
@@ -57,10 +57,10 @@ __global__ void __launch_bounds__(THREADS > 0 ? THREADS : 256) rmsnorm_rope_kern
         const T*    src = qkv + tok * pitch;
         T*          dst = out + tok * pitch;
         // every lane of a warp takes part in the shuffles: those past the end reduce zeros and store nothing
-        for (int v0 = first; v0 - mine < n_vec; v0 += kFlight * step) {
-            uint4 raw[kFlight];
+        for (int v0 = first; v0 - mine < n_vec; v0 += FLIGHT * step) {
+            uint4 raw[FLIGHT];
 #pragma unroll
-            for (int u = 0; u < kFlight; ++u) {
+            for (int u = 0; u < FLIGHT; ++u) {
                 const int vi = v0 + u * step;
                 raw[u] = make_uint4(0u, 0u, 0u, 0u);
                 if (vi < n) {
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(THREADS > 0 ? THREADS : 256) rmsnorm_rope_kern
                 }
             }
 #pragma unroll
-            for (int u = 0; u < kFlight; ++u) {
+            for (int u = 0; u < FLIGHT; ++u) {
                 if (kSplit && u > 0 && v0 - mine + u * step >= n_vec) {
                     break;
                 }
@@ -109,37 +109,45 @@ __global__ void __launch_bounds__(THREADS > 0 ? THREADS : 256) rmsnorm_rope_kern
     }
 }
 
-// Threads of a token.  The q and k heads of 24 x 128 are three vectors for each of 256 threads, with the v heads (out of place) 384, and more
-// heads go through such a block in turns.  With fewer such a block idles, so several tokens share it, still with three vectors a thread:
-// up to 192 vectors always, up to 384 where there are more tokens than blocks.  And where all vectors fit the chip at a few hundred
-// per SM a call is latency: a vector per thread.  Measured against 256 threads to every token and against the flat index: 65536 tokens x
-// 1 head x 64 in place 114 / 12.0 us, here 7.3; 4608 x 2 x 128 10.0 / 4.4, 3.0; 4608 x 12 x 128 12.5 / 15.4, 10.1; out of place 1 x 24 x 128
-// 2.3 / 1.7, 1.75, 77 x 24 x 128 2.7 / 2.7, 2.15, 256 x 24 x 128 3.9 / 3.4, 3.0.
+// Threads of a token.  The q and k heads of 24 x 128 are three vectors for each of 256 threads, with the v heads (out of place) 384: a block
+// a token, three vectors a thread.  Elsewhere such a block idles or takes turns:
+// - up to 1024 threads an SM a call is latency, so every vector gets a thread of a kernel whose code holds one vector only (with room for
+//   three it took 0.1 to 0.25 us of 1.7 more: slower than the flat index).  Not at 257 to 767 vectors, which would double the blocks to save
+//   a second vector: 64 tokens x 12 x 128 out of place 1.94 us so, 1.75 with a block a token;
+// - up to 256 vectors, and up to 384 with many tokens (1024 x 12 x 64 out of place 3.4 us without, 2.75), several tokens share a block;
+// - more than 1152 vectors of few tokens are shared by several blocks.
+// Measured, us, a flat index over all vectors / 256 threads to every token / here: 65536 tokens x 1 head x 64 in place 12.0 / 114 / 7.3; 4608 x
+// 2 x 128 4.4 / 10.0 / 3.0; out of place 1 x 24 x 128 1.6 / 2.3 / 1.45, 128 x 38 x 128 3.25 / 4.2 / 3.0, 256 x 24 x 128 3.2 / 3.9 / 2.8.
 struct RopeSplit {
-    int      threads;            // of the kernel's template: 0, 256 or 384
+    int      threads, flight;    // of the kernel's template: 0 with 1 or 3, 256 or 384 with 3
     int      tpt_log2, chunks;
     unsigned grid;
 };
 static RopeSplit rope_split(size_t tokens, int heads, int lanes, bool in_place, int sms)
 {
     const size_t n_vec = (size_t)heads * (size_t)lanes * (in_place ? 2 : 3);
-    const bool   few   = n_vec <= 192 || (n_vec <= 384 && tokens > (size_t)sms * 8);
-    const bool   brief = few ? n_vec <= 256 && tokens * n_vec <= (size_t)sms * 1024 : n_vec > 768 && tokens * n_vec <= (size_t)sms * 256;
-    RopeSplit    r{0, 3, 1, 0u};
-    size_t       blocks = tokens;
-    if (few || brief) {
-        const size_t want = brief ? n_vec : (n_vec + 2) / 3;
-        while (r.tpt_log2 < 8 && ((1u << r.tpt_log2) < want || (1 << r.tpt_log2) < lanes)) {
+    RopeSplit    r{0, 1, 3, 1, 0u};
+    auto deal = [&](size_t vectors) {   // among 8 .. 256 threads, whole heads, and as many blocks as that takes
+        r.tpt_log2 = 3;
+        while (r.tpt_log2 < 8 && ((size_t)1 << r.tpt_log2 < vectors || (1 << r.tpt_log2) < lanes)) {
             ++r.tpt_log2;
         }
-        const size_t at_once = 256u >> r.tpt_log2;
-        blocks               = (tokens + at_once - 1) / at_once;
-        r.chunks             = brief ? (int)((n_vec + 255) / 256) : 1;
-    } else {
-        r.threads = n_vec > 768 && n_vec <= 1152 ? 384 : 256;
+        r.chunks = (int)((vectors + 255) / 256);
+    };
+    deal(n_vec);
+    if ((n_vec > 256 && n_vec < 768) || (tokens << r.tpt_log2) * (size_t)r.chunks > (size_t)sms * 1024) {
+        r.flight = 3;
+        if (n_vec <= 256 || (n_vec <= 384 && tokens > (size_t)sms * 4) || (n_vec > 1152 && tokens <= (size_t)sms * 2)) {
+            deal((n_vec + 2) / 3);
+        } else {
+            r.threads = n_vec > 768 && n_vec <= 1152 ? 384 : 256;
+            r.chunks  = 1;
+        }
     }
-    const size_t most = (size_t)sms * 8;
-    r.grid            = (unsigned)((blocks < most ? blocks : most) * (size_t)r.chunks);
+    const size_t at_once = r.threads > 0 ? 1 : 256u >> r.tpt_log2;
+    const size_t blocks  = (tokens + at_once - 1) / at_once;
+    const size_t most    = (size_t)sms * 8;
+    r.grid               = (unsigned)((blocks < most ? blocks : most) * (size_t)r.chunks);
     return r;
 }
 
@@ -282,9 +290,10 @@ int lyraq_rmsnorm_rope(void* out, const void* qkv, const void* scale, const void
     auto pick = [&](auto type, auto lanes) {
         using T             = decltype(type);
         constexpr int kLanes = decltype(lanes)::value;
-        return split.threads == 0     ? launch(rmsnorm_rope_kernel<T, kLanes, 0>, type)
-               : split.threads == 256 ? launch(rmsnorm_rope_kernel<T, kLanes, 256>, type)
-                                      : launch(rmsnorm_rope_kernel<T, kLanes, 384>, type);
+        return split.flight == 1      ? launch(rmsnorm_rope_kernel<T, kLanes, 0, 1>, type)
+               : split.threads == 0   ? launch(rmsnorm_rope_kernel<T, kLanes, 0, 3>, type)
+               : split.threads == 256 ? launch(rmsnorm_rope_kernel<T, kLanes, 256, 3>, type)
+                                      : launch(rmsnorm_rope_kernel<T, kLanes, 384, 3>, type);
     };
     auto pick_lanes = [&](auto type) {
         return head_dim == 128 ? pick(type, std::integral_constant<int, 16>{}) : pick(type, std::integral_constant<int, 8>{});

@@ -45,10 +45,11 @@ def test_rmsnorm_rope_against_oracle(ops, dtype, batch, seq, heads, head_dim):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("tokens,heads,head_dim", [(6501, 1, 64), (2501, 2, 128), (2501, 8, 128), (1301, 12, 128), (2501, 24, 128), (5, 30, 128),
-                                                   (3, 130, 64), (1190, 33, 128)])
+                                                   (3, 130, 64), (1190, 33, 128), (150, 38, 128), (701, 12, 64), (1023, 3, 128)])
 def test_rmsnorm_rope_threads_of_a_token(ops, dtype, tokens, heads, head_dim):
     """Every way to deal a token's heads to threads: several tokens to a warp and to a block, a token to a block of either size with more
-    tokens than blocks, a token over several blocks; token counts that fill neither a block nor a round of them.  Bounds as above."""
+    tokens than blocks, a token over several blocks with one vector or three a thread; token counts that fill neither a block nor a round
+    of them.  Bounds as above."""
     test_rmsnorm_rope_against_oracle(ops, dtype, 1, tokens, heads, head_dim)
 
 
